@@ -85,7 +85,8 @@ extern "C" int b200sa_rotor_anneal(int32_t num_vars, const double *h, int64_t nu
     DevArray<int32_t> dcol, dcu, dcv;
     DevArray<double> dw, dh, dtf, dcw, dhp, dhd, dde, den, dtab;
     DevArray<uint64_t> dseeds;
-    DevArray<uint8_t> dst, drows, dstats;
+    DevArray<uint8_t> dst, drows, dstats, ddist;
+    DevArray<uint32_t> dshare, dtouch;
     DevArray<unsigned long long> dnear;
     std::vector<uint2> vinfo(n);
     for (size_t v = 0; v < n; ++v)
@@ -105,9 +106,9 @@ extern "C" int b200sa_rotor_anneal(int32_t num_vars, const double *h, int64_t nu
     B200SA_CUDA(dhd.alloc(std::max<size_t>((size_t)num_betas, 1)));
     B200SA_CUDA(dtab.alloc(512));
     B200SA_CUDA(dseeds.alloc((size_t)num_seeds));
-    B200SA_CUDA(dst.alloc(n * R));
     B200SA_CUDA(drows.alloc(n * R));
-    B200SA_CUDA(dde.alloc(n * R));
+    B200SA_CUDA(ddist.alloc(n));
+    B200SA_CUDA(dshare.alloc(n));
     B200SA_CUDA(den.alloc(R));
     B200SA_CUDA(dnear.alloc(1));
     if (statistics && points) B200SA_CUDA(dstats.alloc(R * (size_t)points * n));
@@ -126,6 +127,9 @@ extern "C" int b200sa_rotor_anneal(int32_t num_vars, const double *h, int64_t nu
     B200SA_CUDA(up(dhd.ptr, hd_field, 8 * (size_t)num_betas));
     B200SA_CUDA(up(dtab.ptr, tab.data(), 8 * 512));
     B200SA_CUDA(up(dseeds.ptr, seeds, 8 * (size_t)num_seeds));
+    B200SA_CUDA(up(ddist.ptr, adj.dist.data(), n));
+    B200SA_CUDA(up(dshare.ptr, adj.share.data(), 4 * n));
+    B200SA_CUDA(upload_jump_table(jump_table(), nullptr));
     B200SA_CUDA(up(drows.ptr, states, n * R));
     B200SA_CUDA(cudaMemset(dnear.ptr, 0, sizeof(unsigned long long)));
     RmcArgs a{};
@@ -147,20 +151,70 @@ extern "C" int b200sa_rotor_anneal(int32_t num_vars, const double *h, int64_t nu
     a.shared_stream = shared ? 1 : 0;
     a.num_samples = num_samples;
     a.rows = drows.ptr;
-    a.states = dst.ptr;
-    a.de = dde.ptr;
+    a.dist = ddist.ptr;
+    a.share = dshare.ptr;
+    a.regular_degree = adj.regular_degree;
+    a.regular_magic = adj.regular_degree ? (65536u + (uint32_t)adj.regular_degree - 1) /
+                                               (uint32_t)adj.regular_degree
+                                         : 0u;
     a.energies = den.ptr;
     a.stats = (statistics && points) ? dstats.ptr : nullptr;
     a.interval = schedule_sample_interval;
     a.cos_table = dtab.ptr;
     a.sin_table = dtab.ptr + 256;
     a.near = dnear.ptr;
-    // Each read is one latency-bound chain: small CTAs spread the reads over
-    // every SM (up to 32 CTAs per SM); 64-thread CTAs once the reads fill them.
+    // One warp per sample, or one thread with very many samples of the
+    // proposals that keep no delta energies (see rmc_kernel.cuh).  A warp's
+    // state is on chip while that keeps 12 warps per SM, or a warp for every
+    // sample; otherwise delta energies, and last the angles, go to per-warp
+    // global slots.  At equal residency the widest CTA is taken, narrower ones
+    // only to spread few samples over every SM.
+    const bool random = randomize_order != 0;
+    const bool threads = proposal >= 2 && !shared && (int64_t)R > kRmcThreadSamples;
     const int sms = prop.multiProcessorCount;
-    const int block = R >= (size_t)sms * 32 * 64 ? 64 : 32;
-    const int grid = shared ? 1 : (int)((R + block - 1) / block);
-    B200SA_CUDA(launch_rmc(randomize_order != 0, proposal, a, grid, block, nullptr));
+    const int64_t chains = shared ? 1 : (int64_t)R;
+    // (A bitmap of more than 256 Ki variables stays in global memory.)
+    a.touch_bytes = touch_bytes_for(random, num_vars);
+    const int touch_region = a.touch_bytes <= 32 * 1024 ? a.touch_bytes : 0;
+    if (threads) {
+        B200SA_CUDA(dst.alloc(n * R));
+        a.states = dst.ptr;
+        B200SA_CUDA(launch_rmc_thread(random, proposal, a, nullptr));
+    } else {
+        int stage = kStageGlobal, width = 1, ctas = 1;
+        for (const int st : {(int)kStageShared, (int)kStageSpins, (int)kStageGlobal}) {
+            if (st == kStageShared && proposal >= 2) continue;  // no delta energies
+            const int64_t region = rmc_region_bytes(st, num_vars, touch_region);
+            if (kRmcTableBytes + region > (int64_t)prop.sharedMemPerBlockOptin) continue;
+            int best = 0;
+            for (int w = 1; w <= kRmcMaxWarps; ++w) {
+                if (kRmcTableBytes + w * region > (int64_t)prop.sharedMemPerBlockOptin) break;
+                int c = 0;
+                B200SA_CUDA(rmc_occupancy(random, proposal, st, w, region, &c));
+                if (c * w >= best) best = c * w, width = w, ctas = c;
+                if ((int64_t)sms * w >= chains) break;
+            }
+            stage = st;
+            if (best >= 12 || (best > 0 && (int64_t)sms * best >= chains)) break;
+        }
+        a.region_bytes = (int32_t)rmc_region_bytes(stage, num_vars, touch_region);
+        const int grid = (int)std::max<int64_t>(
+            1, std::min<int64_t>((int64_t)sms * ctas, (chains + width - 1) / width));
+        if (shared) width = 1;
+        if (a.touch_bytes != touch_region) {
+            B200SA_CUDA(dtouch.alloc((size_t)grid * (size_t)width * (size_t)(a.touch_bytes / 4)));
+            a.touch = dtouch.ptr;
+        }
+        if (stage != kStageShared) {
+            a.slot_stride = (int64_t)((n + 15) & ~size_t(15));
+            const size_t elems = (size_t)grid * (size_t)width * (size_t)a.slot_stride;
+            if (proposal <= 1) B200SA_CUDA(dde.alloc(elems));
+            if (stage == kStageGlobal) B200SA_CUDA(dst.alloc(elems));
+            a.de = dde.ptr;
+            a.states = dst.ptr;
+        }
+        B200SA_CUDA(launch_rmc(random, proposal, stage, a, grid, width, nullptr));
+    }
     B200SA_CUDA(cudaDeviceSynchronize());
     B200SA_CUDA(cudaMemcpy(states, drows.ptr, n * R, cudaMemcpyDeviceToHost));
     B200SA_CUDA(cudaMemcpy(energies, den.ptr, 8 * R, cudaMemcpyDeviceToHost));

@@ -438,21 +438,19 @@ __device__ __forceinline__ void add_group(const DE &de, int x, unsigned grp, con
     }
 }
 
-// cpu_sa.cpp:168-191 for every lane whose bit is set in `fm`.  Lane k of
-// the warp holds its variable v, list start `start`, degree `deg` and spin
-// `s_old` (valid on flipping lanes).  The flipping variables must be pairwise
+// The neighbour updates of every lane whose bit is set in `fm`: slot x gets
+// (mult * J) * val(x) for each entry (x, J) of the lane's list.  Lane k of the
+// warp holds its variable v, list start `start`, degree `deg` and factor
+// `mult` (valid on flipping lanes).  The flipping variables must be pairwise
 // non-adjacent.  Entries are applied lane-parallel in rounds of 32; equal
 // targets within a round are summed in entry order by their first lane.
-// `scratch` holds 32 doubles followed by 32 ints.  With `own_fresh`, no entry
-// of this pass names the lane's own slot, which then still holds `d_own`.
-template <class DE>
-__device__ __forceinline__ void apply_flips(const Prob &P, DE de, int8_t *sp,
-                                            double *scratch, unsigned fm, int v,
-                                            int start, int deg, int s_old,
-                                            bool may_conflict, unsigned lane,
-                                            bool own_fresh = false, double d_own = 0.0) {
+// `scratch` holds 32 doubles followed by 32 ints.
+template <class DE, class VAL>
+__device__ __forceinline__ void push_entries(const Prob &P, DE de, VAL val,
+                                             double *scratch, unsigned fm, int v,
+                                             int start, int deg, double mult,
+                                             bool may_conflict, unsigned lane) {
     const bool f = (fm >> lane) & 1u;
-    const double mult = (double)(int)(int8_t)(4 * s_old);
     int *owner_of_rank = reinterpret_cast<int *>(scratch + 32);
     const int D = P.regular_degree;
     int excl = 0, total;
@@ -493,7 +491,7 @@ __device__ __forceinline__ void apply_flips(const Prob &P, DE de, int8_t *sp,
                 x[i] = 0.0;
                 if (t < total) {
                     nb[i] = __ldg(&P.col[e]);
-                    x[i] = __dmul_rn(__dmul_rn(m_k, __ldg(&P.w[e])), (double)(int)sp[nb[i]]);
+                    x[i] = __dmul_rn(__dmul_rn(m_k, __ldg(&P.w[e])), val(nb[i]));
                 }
             }
             if constexpr (DE::kAsyncAdd) {
@@ -535,7 +533,7 @@ __device__ __forceinline__ void apply_flips(const Prob &P, DE de, int8_t *sp,
         double x = 0.0;
         if (a) {
             nb = __ldg(&P.col[e]);
-            x = __dmul_rn(__dmul_rn(m_k, __ldg(&P.w[e])), (double)(int)sp[nb]);
+            x = __dmul_rn(__dmul_rn(m_k, __ldg(&P.w[e])), val(nb));
         }
         const unsigned grp = may_conflict ? __match_any_sync(kFull, nb) : (1u << lane);
         const bool alone = grp == (1u << lane);
@@ -549,7 +547,20 @@ __device__ __forceinline__ void apply_flips(const Prob &P, DE de, int8_t *sp,
         }
         __syncwarp();
     }
-    if (f) {  // cpu_sa.cpp:189-190, after the variable's own updates
+}
+
+// cpu_sa.cpp:168-191 for the flips `fm` (see push_entries); `s_old` is the
+// lane's spin.  With `own_fresh`, no entry of this pass names the lane's own
+// slot, which then still holds `d_own`.
+template <class DE>
+__device__ __forceinline__ void apply_flips(const Prob &P, DE de, int8_t *sp,
+                                            double *scratch, unsigned fm, int v,
+                                            int start, int deg, int s_old,
+                                            bool may_conflict, unsigned lane,
+                                            bool own_fresh = false, double d_own = 0.0) {
+    push_entries(P, de, [&](int x) { return (double)(int)sp[x]; }, scratch, fm, v, start, deg,
+                 (double)(int)(int8_t)(4 * s_old), may_conflict, lane);
+    if ((fm >> lane) & 1u) {  // cpu_sa.cpp:189-190, after the variable's own updates
         sp[v] = (int8_t)(-s_old);
         de.set(v, __dmul_rn(own_fresh ? d_own : de.get(v), -1.0));
     }
@@ -1020,6 +1031,96 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
     }
 }
 
+// rv % n (cpu_sa.cpp:135) with magic = (2^64 - 1) / n: the estimated quotient
+// is at most one too small.
+__device__ __forceinline__ int mod_n(uint64_t rv, uint32_t n, uint64_t magic) {
+    const uint64_t r = rv - __umul64hi(rv, magic) * (uint64_t)n;
+    return (int)(uint32_t)(r >= n ? r - n : r);
+}
+
+// Lists up to this long are scanned by their own lane for the window's
+// accepted variables (random_commit).
+constexpr int kScanDegree = 24;
+
+// The commit point of a window in random order: the first chain lane whose
+// variable an earlier accepted lane (bit of A) flipped or neighbours; 32 when
+// there is none.  `touch` is a bitmap of the variables, clear before and after.
+//
+// Short lists: the accepted lanes mark their variables all at once and every
+// chain lane looks for a mark in its own list, so a window without a hit (the
+// usual one on a sparse graph) costs one scan, whatever the number of
+// accepted lanes; only then are the accepted lanes gone through in order.
+// Long lists: the accepted lanes mark their neighbours one after another, the
+// list spread over the warp.
+__device__ __forceinline__ int random_commit(const Prob &P, int D, uint32_t *touch, int var,
+                                             bool chain, unsigned A, unsigned lane) {
+    if (!A) return 32;
+    const uint2 own = D ? make_uint2((uint32_t)var * (uint32_t)D, (uint32_t)D)
+                        : __ldg(&P.vinfo[var]);
+    const unsigned deg_own = own.y & kDegMask;
+    const bool acc = (A >> lane) & 1u;
+    int c = 32;
+    if (__all_sync(kFull, deg_own <= (unsigned)kScanDegree)) {
+        if (acc) atomicOr(&touch[var >> 5], 1u << (var & 31));
+        __syncwarp();
+        bool near = false;
+        for (unsigned t = 0; t < deg_own; ++t) {
+            const int x = __ldg(&P.col[own.x + t]);
+            near = near || ((touch[x >> 5] >> (x & 31)) & 1u);
+        }
+        const unsigned lt_mask = (1u << lane) - 1u;
+        const bool again = (__match_any_sync(kFull, var) & A & lt_mask) != 0u;
+        __syncwarp();
+        if (acc) touch[var >> 5] = 0u;
+        const unsigned H = __ballot_sync(kFull, chain && again);
+        if (H) c = __ffs(H) - 1;
+        const unsigned M = __ballot_sync(kFull, chain && near);
+        if (M & ((c >= 32 ? kFull : (1u << c) - 1u))) {
+            for (unsigned todo = A; todo; todo &= todo - 1u) {
+                const int j = __ffs(todo) - 1;
+                if (j >= c) break;
+                const int vj = __shfl_sync(kFull, var, j);
+                bool hit = false;
+                if (chain && near && (int)lane > j)
+                    for (unsigned t = 0; t < deg_own && !hit; ++t)
+                        hit = __ldg(&P.col[own.x + t]) == vj;
+                const unsigned h = __ballot_sync(kFull, hit);
+                if (h) c = min(c, __ffs(h) - 1);
+            }
+        }
+        __syncwarp();
+        return c;
+    }
+    unsigned todo = A, marked = 0u;
+    while (todo) {
+        const int j = __ffs(todo) - 1;
+        if (j >= c) break;
+        todo &= todo - 1u;
+        marked |= 1u << j;
+        const int vj = __shfl_sync(kFull, var, j);
+        const unsigned start = __shfl_sync(kFull, own.x, j), deg = __shfl_sync(kFull, deg_own, j);
+        for (unsigned t = lane; t < deg; t += 32) {
+            const int x = __ldg(&P.col[start + t]);
+            atomicOr(&touch[x >> 5], 1u << (x & 31));
+        }
+        if (lane == 0) atomicOr(&touch[vj >> 5], 1u << (vj & 31));
+        __syncwarp();
+        const bool hit = chain && (int)lane > j && ((touch[var >> 5] >> (var & 31)) & 1u);
+        const unsigned H = __ballot_sync(kFull, hit);
+        if (H) c = min(c, __ffs(H) - 1);
+    }
+    __syncwarp();
+    for (unsigned m = marked; m; m &= m - 1u) {  // clear the marked words for the next pass
+        const int j = __ffs(m) - 1;
+        const int vj = __shfl_sync(kFull, var, j);
+        const unsigned start = __shfl_sync(kFull, own.x, j), deg = __shfl_sync(kFull, deg_own, j);
+        for (unsigned t = lane; t < deg; t += 32) touch[__ldg(&P.col[start + t]) >> 5] = 0u;
+        if (lane == 0) touch[vj >> 5] = 0u;
+    }
+    __syncwarp();
+    return c;
+}
+
 // Random order (cpu_sa.cpp:134-139) in speculative windows of the RNG
 // stream.  Each attempt draws its variable as rand % n and, when it needs one,
 // its acceptance draw right after it.  Lane l takes stream position q + l as
@@ -1082,45 +1183,7 @@ __device__ __forceinline__ void sweep_random(const Prob &P, DE de,
                     }
                 }
                 const unsigned A = __ballot_sync(kFull, acc);
-                // Commit point: the first chain lane whose variable an earlier
-                // accepted flip touched.  Accepted lanes are marked in order.
-                int c = 32;
-                unsigned todo = A, marked = 0u;
-                while (todo) {
-                    const int j = __ffs(todo) - 1;
-                    if (j >= c) break;
-                    todo &= todo - 1u;
-                    marked |= 1u << j;
-                    const int vj = __shfl_sync(kFull, var, j);
-                    const uint2 vi = D ? make_uint2((uint32_t)vj * (uint32_t)D, (uint32_t)D)
-                                       : __ldg(&P.vinfo[vj]);
-                    const int deg = (int)(vi.y & kDegMask);
-                    for (int t = (int)lane; t < deg; t += 32) {
-                        const int x = __ldg(&P.col[vi.x + (uint32_t)t]);
-                        atomicOr(&touch[x >> 5], 1u << (x & 31));
-                    }
-                    if (lane == 0) atomicOr(&touch[vj >> 5], 1u << (vj & 31));
-                    __syncwarp();
-                    const bool hit = chain && (int)lane > j && ((touch[var >> 5] >> (var & 31)) & 1u);
-                    const unsigned H = __ballot_sync(kFull, hit);
-                    if (H) c = min(c, __ffs(H) - 1);
-                }
-                if (marked) {  // clear the marked words for the next pass
-                    __syncwarp();
-                    unsigned m = marked;
-                    while (m) {
-                        const int j = __ffs(m) - 1;
-                        m &= m - 1u;
-                        const int vj = __shfl_sync(kFull, var, j);
-                        const uint2 vi = D ? make_uint2((uint32_t)vj * (uint32_t)D, (uint32_t)D)
-                                           : __ldg(&P.vinfo[vj]);
-                        const int deg = (int)(vi.y & kDegMask);
-                        for (int t = (int)lane; t < deg; t += 32)
-                            touch[__ldg(&P.col[vi.x + (uint32_t)t]) >> 5] = 0u;
-                        if (lane == 0) touch[vj >> 5] = 0u;
-                    }
-                    __syncwarp();
-                }
+                const int c = random_commit(P, D, touch, var, chain, A, lane);
                 const unsigned cm = C & (c >= 32 ? kFull : ((1u << c) - 1u));
                 const int last = 31 - __clz(cm);  // lane 0 is always committed
                 rs.q += (uint32_t)(last + 1) + ((N >> last) & 1u);

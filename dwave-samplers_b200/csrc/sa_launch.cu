@@ -289,14 +289,55 @@ cudaError_t sd_occupancy(bool sparse, bool smem, int warps_per_cta, int region_b
 
 using RmcKernel = void (*)(RmcArgs);
 
-cudaError_t launch_rmc(bool random_order, int proposal, const RmcArgs &args, int grid,
-                       int block, cudaStream_t stream) {
-    static const RmcKernel table[2][4] = {
-        {rmc_kernel<false, 0>, rmc_kernel<false, 1>, rmc_kernel<false, 2>, rmc_kernel<false, 3>},
-        {rmc_kernel<true, 0>, rmc_kernel<true, 1>, rmc_kernel<true, 2>, rmc_kernel<true, 3>}};
-    if (proposal < 0 || proposal > 3) return cudaErrorInvalidValue;
-    table[random_order ? 1 : 0][proposal]<<<grid, block, 0, stream>>>(args);
+#define B200SA_RMC_STAGES(order, proposal)                                            \
+    {rmc_kernel<order, proposal, kStageGlobal>,                                       \
+     rmc_kernel<order, proposal, (proposal) <= 1 ? kStageShared : kStageSpins>,       \
+     rmc_kernel<order, proposal, kStageSpins>}
+#define B200SA_RMC_PROPOSALS(order)                                                   \
+    {B200SA_RMC_STAGES(order, 0), B200SA_RMC_STAGES(order, 1), B200SA_RMC_STAGES(order, 2), \
+     B200SA_RMC_STAGES(order, 3)}
+
+static RmcKernel rmc_kernel_for(bool random_order, int proposal, int stage) {
+    static const RmcKernel table[2][4][3] = {B200SA_RMC_PROPOSALS(false),
+                                             B200SA_RMC_PROPOSALS(true)};
+    if (proposal < 0 || proposal > 3 || stage < 0 || stage > kStageSpins) return nullptr;
+    if (proposal >= 2 && stage == kStageShared) return nullptr;
+    return table[random_order ? 1 : 0][proposal][stage];
+}
+
+static cudaError_t rmc_smem(RmcKernel k, int warps_per_cta, int64_t region_bytes, size_t &smem) {
+    if (!k) return cudaErrorInvalidValue;
+    smem = (size_t)kRmcTableBytes + (size_t)warps_per_cta * (size_t)region_bytes;
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
+
+cudaError_t launch_rmc(bool random_order, int proposal, int stage, const RmcArgs &args, int grid,
+                       int warps_per_cta, cudaStream_t stream) {
+    const RmcKernel k = rmc_kernel_for(random_order, proposal, stage);
+    size_t smem = 0;
+    const cudaError_t e = rmc_smem(k, warps_per_cta, args.region_bytes, smem);
+    if (e != cudaSuccess) return e;
+    k<<<grid, warps_per_cta * 32, smem, stream>>>(args);
     return cudaGetLastError();
+}
+
+cudaError_t launch_rmc_thread(bool random_order, int proposal, const RmcArgs &args,
+                              cudaStream_t stream) {
+    static const RmcKernel table[2][2] = {{rmc_thread_kernel<false, 2>, rmc_thread_kernel<false, 3>},
+                                          {rmc_thread_kernel<true, 2>, rmc_thread_kernel<true, 3>}};
+    if (proposal != 2 && proposal != 3) return cudaErrorInvalidValue;
+    const int64_t grid = ((int64_t)args.num_samples + 63) / 64;
+    table[random_order ? 1 : 0][proposal - 2]<<<(unsigned)grid, 64, 0, stream>>>(args);
+    return cudaGetLastError();
+}
+
+cudaError_t rmc_occupancy(bool random_order, int proposal, int stage, int warps_per_cta,
+                          int64_t region_bytes, int *ctas_per_sm) {
+    const RmcKernel k = rmc_kernel_for(random_order, proposal, stage);
+    size_t smem = 0;
+    const cudaError_t e = rmc_smem(k, warps_per_cta, region_bytes, smem);
+    if (e != cudaSuccess) return e;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, k, warps_per_cta * 32, smem);
 }
 
 cudaError_t launch_pimc(bool chain_update, const PimcArgs &args, int grid, int block,

@@ -42,8 +42,15 @@ cudaError_t launch_sd(bool sparse, bool smem, const SdArgs &args, int grid, int 
                       int region_bytes, cudaStream_t stream);
 cudaError_t sd_occupancy(bool sparse, bool smem, int warps_per_cta, int region_bytes,
                          int *ctas_per_sm);
-cudaError_t launch_rmc(bool random_order, int proposal, const RmcArgs &args, int grid,
-                       int block, cudaStream_t stream);
+// Rotor kernel; `stage` is its state location (kStageShared only for the
+// proposals that keep delta energies, 0 and 1).
+cudaError_t launch_rmc(bool random_order, int proposal, int stage, const RmcArgs &args, int grid,
+                       int warps_per_cta, cudaStream_t stream);
+// One thread per sample (proposals 2 and 3).
+cudaError_t launch_rmc_thread(bool random_order, int proposal, const RmcArgs &args,
+                              cudaStream_t stream);
+cudaError_t rmc_occupancy(bool random_order, int proposal, int stage, int warps_per_cta,
+                          int64_t region_bytes, int *ctas_per_sm);
 cudaError_t launch_pimc(bool chain_update, const PimcArgs &args, int grid, int block,
                         cudaStream_t stream);
 cudaError_t acceptance_check(int64_t samples, uint64_t seed, unsigned long long *d_counts);

@@ -160,14 +160,31 @@ struct RmcArgs {
     int32_t shared_stream;   // 1: one thread, samples in order, one RNG stream
     int32_t num_samples;
     uint8_t *rows;           // [num_samples][n] initial states in, final states out
-    uint8_t *states;         // working copy, interleaved: element (v, r) at v * num_samples + r
-    double *de;              // interleaved like states
+    const uint8_t *dist;     // [n] speculation distance (ProblemDev::dist)
+    const uint32_t *share;   // [n] conflict mask (ProblemDev::share)
+    int32_t regular_degree;  // ProblemDev::regular_degree, regular_magic
+    uint32_t regular_magic;
+    int32_t region_bytes;    // a warp's shared region (rmc_region_bytes)
+    int32_t touch_bytes;     // random order: bytes of a warp's touch bitmap
+    uint32_t *touch;         // the bitmaps, one per warp, or null: in the region
+    double *de;              // per-warp global slots of slot_stride elements
+    uint8_t *states;         // (state locations kStageSpins and kStageGlobal);
+    int64_t slot_stride;     // one thread per sample: angles, [n][num_samples]
     double *energies;
     uint8_t *stats;          // [num_samples][points][n], or null
     int32_t interval;
     const double *cos_table, *sin_table;  // [256]
     unsigned long long *near;
 };
+
+// Shared memory of the rotor kernel: the two angle tables per CTA, then per
+// warp the RNG ring, scratch, touch bitmap and, by the state location, delta
+// energies (proposals that keep them) and angles.
+constexpr int kRmcTableBytes = 2 * 256 * 8;
+constexpr int kRmcMaxWarps = 8;  // warps per CTA
+// Above this many samples the uniform and transverse-field proposals run one
+// thread per sample (both sides measured, see rmc_kernel.cuh).
+constexpr int64_t kRmcThreadSamples = 16384;
 
 // Arguments of the path-integral Monte Carlo kernel (pimc_kernel.cuh).  One
 // thread per sample (a "slot"); every slot owns an mt19937 state and a
@@ -248,6 +265,14 @@ inline int region_bytes_for_stage(int stage, int cap_n, int band_cap = 0) {
     if (stage == kStageSpins) return kRing * 8 + kScratchBytes + ((cap_n + 15) & ~15);
     if (stage == kStageBand) return kRing * 8 + kScratchBytes + ((cap_n + 15) & ~15) + 8 * band_cap;
     return kRing * 8 + kScratchBytes;
+}
+
+// Rotor kernel: kStageShared delta energies and angles, kStageSpins angles,
+// kStageGlobal neither.
+inline int64_t rmc_region_bytes(int stage, int64_t n, int touch_bytes) {
+    const int64_t angles = (n + 15) & ~int64_t(15);
+    return kRing * 8 + kScratchBytes + touch_bytes + (stage != kStageGlobal ? angles : 0) +
+           (stage == kStageShared ? (n * 8 + 15) & ~int64_t(15) : 0);
 }
 
 // Random order keeps a bitmap of n bits per warp (16-byte multiple).
