@@ -83,6 +83,7 @@ extern "C" int b200sa_path_anneal(
     const size_t n = (size_t)num_vars, R = (size_t)num_samples, m = (size_t)num_couplers;
     // Quantum initial states: num_breaks[r][v] positions per variable, in order.
     int max_in = 0;
+    bool ordered = true;  // every list increasing, within the slices
     if (!project_inputs) {
         int64_t total = 0;
         for (size_t i = 0; i < R * n; ++i) {
@@ -94,9 +95,21 @@ extern "C" int b200sa_path_anneal(
         if (total > breaks_in_size || (total > 0 && !breaks_in))
             return set_err(err, errlen, B200SA_EINVAL,
                            "breaks_in holds fewer positions than num_breaks asks for");
+        int64_t pos = 0;
+        for (size_t i = 0; i < R * n; ++i)
+            for (int32_t k = 0, prev = 0; k < num_breaks[i]; ++k) {
+                const int32_t b = breaks_in[pos++];
+                ordered = ordered && b >= prev && b < kPimcSlices;
+                prev = b;
+            }
     }
     const int cap_props = break_capacity ? break_capacity : auto_capacity(hd_field, num_betas);
     const int cap_breaks = std::max(cap_props, (max_in + 3) & ~3);
+    // Single-qubit updates run on a warp per sample while a CTA's warps fit in
+    // shared memory; chain updates, very large capacities and break lists out
+    // of order on one thread per sample.
+    const int64_t warp_bytes = pimc_warp_bytes(cap_props, cap_breaks);
+    const bool warp = !chain && ordered && warp_bytes <= 48 * 1024;
     const int Q = chain ? qubits_per_chain : 1;
     const int64_t C = (int64_t)cap_props + cap_breaks;
     // props, itf [Q][C], sv [Q * C], off [Q + 1], lab [Q * C], parent [Q * C], pair [2C]
@@ -141,7 +154,8 @@ extern "C" int b200sa_path_anneal(
     DevArray<uint32_t> dseeds, dmt;
     DevArray<int8_t> dst, dstats;
     DevArray<unsigned long long> dnear;
-    const size_t list_words = R * n * (size_t)cap_breaks;
+    const size_t list_stride = ((size_t)cap_breaks + 3) & ~size_t(3);
+    const size_t list_words = R * n * list_stride;
     B200SA_CUDA(dvinfo.alloc(n));
     B200SA_CUDA(dcol.alloc(std::max<size_t>(2 * m, 1)));
     B200SA_CUDA(dw.alloc(std::max<size_t>(2 * m, 1)));
@@ -155,9 +169,11 @@ extern "C" int b200sa_path_anneal(
     B200SA_CUDA(dst.alloc(n * R));
     B200SA_CUDA(dcnt.alloc(n * R));
     B200SA_CUDA(dbrk.alloc(list_words));
-    B200SA_CUDA(dmt.alloc(slots * kMtWords));
-    B200SA_CUDA(dscr_i.alloc(slots * (size_t)scratch_ints));
-    B200SA_CUDA(dscr_d.alloc(slots * (size_t)scratch_doubles));
+    if (!warp) {
+        B200SA_CUDA(dmt.alloc(slots * kMtWords));
+        B200SA_CUDA(dscr_i.alloc(slots * (size_t)scratch_ints));
+        B200SA_CUDA(dscr_d.alloc(slots * (size_t)scratch_doubles));
+    }
     B200SA_CUDA(den.alloc(R));
     B200SA_CUDA(dnear.alloc(1));
     B200SA_CUDA(dflag.alloc(1));
@@ -183,7 +199,7 @@ extern "C" int b200sa_path_anneal(
         size_t pos = 0;
         for (size_t i = 0; i < R * n; ++i)
             for (int k = 0; k < num_breaks[i]; ++k)
-                lists[i * (size_t)cap_breaks + k] = breaks_in[pos++];
+                lists[i * list_stride + k] = breaks_in[pos++];
         B200SA_CUDA(up(dcnt.ptr, num_breaks, 4 * n * R));
         B200SA_CUDA(up(dbrk.ptr, lists.data(), 4 * list_words));
     }
@@ -213,6 +229,7 @@ extern "C" int b200sa_path_anneal(
     a.counts = dcnt.ptr;
     a.breaks = dbrk.ptr;
     a.cap_breaks = cap_breaks;
+    a.list_stride = (int32_t)list_stride;
     a.cap_props = cap_props;
     a.mt = dmt.ptr;
     a.scratch_i = dscr_i.ptr;
@@ -224,12 +241,17 @@ extern "C" int b200sa_path_anneal(
     a.interval = schedule_sample_interval;
     a.near = dnear.ptr;
     a.overflow = dflag.ptr;
-    // One latency-bound chain per sample: small CTAs spread the samples over
-    // every SM.
     const int sms = prop.multiProcessorCount;
-    const int block = R >= (size_t)sms * 32 * 64 ? 64 : 32;
-    const int grid = shared ? 1 : (int)((R + block - 1) / block);
-    B200SA_CUDA(launch_pimc(chain, a, grid, block, nullptr));
+    if (warp) {  // few samples: narrow CTAs, spread over every SM
+        const int64_t chains = shared ? 1 : (int64_t)R;
+        const int w = (int)std::min<int64_t>(kPimcMaxWarps, (chains + sms - 1) / sms);
+        B200SA_CUDA(launch_pimc_warp(a, (int)((chains + w - 1) / w), w, (int)warp_bytes, nullptr));
+    } else {
+        // One thread per sample: small CTAs spread the samples over every SM.
+        const int block = R >= (size_t)sms * 32 * 64 ? 64 : 32;
+        const int grid = shared ? 1 : (int)((R + block - 1) / block);
+        B200SA_CUDA(launch_pimc(chain, a, grid, block, nullptr));
+    }
     B200SA_CUDA(cudaDeviceSynchronize());
     int32_t overflow = 0;
     B200SA_CUDA(cudaMemcpy(&overflow, dflag.ptr, sizeof(overflow), cudaMemcpyDeviceToHost));
@@ -260,7 +282,7 @@ extern "C" int b200sa_path_anneal(
             for (size_t v = 0; v < n; ++v) {
                 const int c = num_breaks[r * n + v];
                 if (capacity >= c) {
-                    if (c) std::memcpy(breaks_out + p, &lists[(r * n + v) * (size_t)cap_breaks],
+                    if (c) std::memcpy(breaks_out + p, &lists[(r * n + v) * list_stride],
                                        sizeof(int32_t) * (size_t)c);
                     p += c;
                     capacity -= c;

@@ -349,4 +349,14 @@ cudaError_t launch_pimc(bool chain_update, const PimcArgs &args, int grid, int b
     return cudaGetLastError();
 }
 
+cudaError_t launch_pimc_warp(const PimcArgs &args, int grid, int warps_per_cta, int warp_bytes,
+                             cudaStream_t stream) {
+    const size_t smem = (size_t)warps_per_cta * (size_t)warp_bytes;
+    const cudaError_t e = cudaFuncSetAttribute(
+        pimc_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    pimc_warp_kernel<<<grid, warps_per_cta * 32, smem, stream>>>(args, warp_bytes);
+    return cudaGetLastError();
+}
+
 }  // namespace b200sa

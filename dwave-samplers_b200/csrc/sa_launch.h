@@ -53,6 +53,9 @@ cudaError_t rmc_occupancy(bool random_order, int proposal, int stage, int warps_
                           int64_t region_bytes, int *ctas_per_sm);
 cudaError_t launch_pimc(bool chain_update, const PimcArgs &args, int grid, int block,
                         cudaStream_t stream);
+// Single-qubit updates, one warp per sample.
+cudaError_t launch_pimc_warp(const PimcArgs &args, int grid, int warps_per_cta, int warp_bytes,
+                             cudaStream_t stream);
 cudaError_t acceptance_check(int64_t samples, uint64_t seed, unsigned long long *d_counts);
 
 }  // namespace b200sa

@@ -210,8 +210,9 @@ struct PimcArgs {
     int32_t num_samples;
     int8_t *states;          // [num_samples][n], the first Trotter slice
     int32_t *counts;         // [num_samples][n] breaks per variable
-    int32_t *breaks;         // [num_samples][n][cap_breaks]
+    int32_t *breaks;         // [num_samples][n][list_stride]
     int32_t cap_breaks;
+    int32_t list_stride;     // cap_breaks, rounded up to 16 bytes
     int32_t cap_props;       // proposals per qubit and update
     uint32_t *mt;            // [slots][kMtWords]
     int32_t *scratch_i;      // [slots][scratch_ints]
@@ -224,6 +225,14 @@ struct PimcArgs {
     int32_t *overflow;       // set when a capacity would be exceeded
 };
 constexpr int kMtWords = 624;
+constexpr int kPimcSlices = 65536;  // numTrotterSlices, localPIMC.h:88
+// Warps per CTA of the warp-per-sample kernel at most, and its shared memory
+// per sample: mt19937 state, scratch (PimcWarpScratch).
+constexpr int kPimcMaxWarps = 4;
+inline int64_t pimc_warp_bytes(int64_t cap_props, int64_t cap_breaks) {
+    const int64_t cap = cap_props + cap_breaks;
+    return (4 * kMtWords + 32 * (8 + 4 + 4) + 8 * cap + cap + 15) & ~int64_t(15);
+}
 
 // Nibble tables of the RNG jump matrix: entry [k][v] is the jump applied to
 // the state whose only set bits are the nibble value v at nibble position k.
