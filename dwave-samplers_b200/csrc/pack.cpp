@@ -168,18 +168,25 @@ void pack_adjacency(const b200sa_problem &p, PackedAdjacency &out) {
         out.band_b = b;
         out.band_w = (w <= kBandMaxSlots && 2 * w <= (int64_t)n) ? (int32_t)w : 0;
     }
-    out.dense = out.resolve && n <= kDenseMaxN && 16 * (size_t)m >= (size_t)n * (size_t)n;
+    // State in registers: dense problems (average degree at least n / 8) up to
+    // kDenseMaxN variables, and others while the updates of a whole row cost
+    // less than the general path: 1000 reads x 200 sweeps, n = 60 degree 4 1.22
+    // -> 0.90 ms, n = 120 degree 4 2.02 -> 1.87 and degree 10 2.71 -> 1.55, n =
+    // 250 degree 6 4.15 -> 4.86 (not taken); random order n = 60 4.73 -> 2.00,
+    // n = 120 8.16 -> 4.10, n = 250 14.6 -> 8.6.  Above 64 variables a sparse
+    // problem's matrix is many times its lists, so it is made only for runs long
+    // beside its upload (2^22 attempts, about 0.1 ms).
+    const double attempts = (double)n * p.num_reads * p.sweeps_per_beta * p.num_betas;
+    const bool full = 16 * (size_t)m >= (size_t)n * (size_t)n;
+    const int limit = full || p.varorder == B200SA_RANDOM ? kDenseMaxN : 128;
+    out.dense = !any_dup && n > 0 && n <= limit && (n <= 64 || full || attempts >= 4194304.0);
     out.dense_w.clear();
-    out.dense_bits.clear();
     if (out.dense) {
-        out.dense_w.assign((size_t)n * (size_t)n, 0.0);
-        out.dense_bits.assign((size_t)n * 4, 0u);
+        const size_t ld = (size_t)dense_ld(n);
+        out.dense_w.assign((size_t)n * ld + (size_t)kDenseMaxN, 0.0);
         for (int32_t j = 0; j < n; ++j)
-            for (int32_t e = out.row[j]; e < out.row[j + 1]; ++e) {
-                const int32_t x = out.col[e];
-                out.dense_w[(size_t)j * n + x] = out.w[e];
-                out.dense_bits[(size_t)j * 4 + (x >> 5)] |= 1u << (x & 31);
-            }
+            for (int32_t e = out.row[j]; e < out.row[j + 1]; ++e)
+                out.dense_w[(size_t)j * ld + (size_t)out.col[e]] = out.w[e];
     }
     out.regular_degree = 0;
     if (n > 0 && maxdeg > 0 && maxdeg <= 32) {

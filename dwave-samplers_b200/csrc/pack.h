@@ -26,12 +26,9 @@ struct PackedAdjacency {
     std::vector<double> bw;
     std::vector<int32_t> bw_src;
     bool resolve = false;         // in-window resolution enabled (ProblemDev::resolve)
-    // Dense updates (ProblemDev::dense): n <= 128, average degree >= n/8, no
-    // repeated targets.  dense_w[j*n + x] is the coupling of j and x (0 when
-    // they are not neighbours) and dense_bits[4j .. 4j+3] the 128-bit mask of
-    // j's neighbours.
+    // State in registers (ProblemDev::dense) and its coupling matrix, rows of
+    // dense_ld(n).
     std::vector<double> dense_w;
-    std::vector<uint32_t> dense_bits;
     bool dense = false;
     // Banded delta energies (ProblemDev::band_b / band_w): the smallest
     // offset b >= 32 that covers 97% of the adjacency entries, and the ring

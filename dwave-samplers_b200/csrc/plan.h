@@ -83,8 +83,8 @@ inline void reset_stats(b200sa_stats *s) {
 // Nibble tables of the RNG jump by kHalf outputs (computed once per process).
 const uint32_t (*jump_table())[4];
 
-// Whether plans enable in-window resolution / dense updates for the problems
-// that qualify.
+// Whether plans enable in-window resolution / state in registers / the band
+// for the problems that qualify.
 bool resolve_allowed();
 bool dense_allowed();
 bool band_allowed();
@@ -108,10 +108,10 @@ inline int size_class(int n, int onchip_max) {
 }
 
 // Kernel kind of a problem: bit 0 Gibbs, bit 1 random order, bit 2
-// in-window resolution (sequential order only).
+// in-window resolution (sequential order only), bit 3 state in registers.
 inline int kind_of(const ProblemDev &d) {
     return (d.proposal == 0 ? kKindGibbs : 0) | (d.varorder ? kKindRandom : 0) |
-           (d.resolve && !d.varorder ? kKindResolve : 0);
+           (d.dense ? kKindDense : d.resolve && !d.varorder ? kKindResolve : 0);
 }
 
 // Launch configuration of one bucket chosen by the autotuner (unset: the
@@ -138,7 +138,7 @@ struct LaunchShape {
 
 // Arena byte offsets of one packed problem.
 struct ArenaOffsets {
-    size_t vinfo, dist, share, col, w, h, cu, cv, cw, betas, thr, back, bw, dw, dbits;
+    size_t vinfo, dist, share, col, w, h, cu, cv, cw, betas, thr, back, bw, dw;
 };
 
 }  // namespace host
@@ -175,7 +175,7 @@ struct b200sa_plan_s {
     // Largest band ring of a bucket whose problems are all banded, else 0.
     int32_t bucket_band_w[b200sa::host::kBuckets] = {};
     int64_t bucket_lead_cost[b200sa::host::kBuckets] = {};
-    std::map<std::pair<int, int>, int> occ_cache;  // (variant*2^24 + warps, region) -> CTAs/SM
+    std::map<std::pair<int, int>, int> occ_cache;  // (variant*2^8 + warps, region) -> CTAs/SM
     int64_t launches = 0;  // sweep-kernel launches issued by the current run
     std::vector<b200sa::host::ArenaOffsets> offs;  // per problem
     std::vector<std::vector<int32_t>> rows;        // per problem: CSR list starts (n + 1)

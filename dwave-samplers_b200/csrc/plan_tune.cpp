@@ -327,10 +327,11 @@ int b200sa_plan_set_weights(b200sa_plan plan, int32_t problem, const double *h, 
     // couplers there, so each entry is one coupler's weight).
     std::vector<double> dw;
     if (d.dense) {
-        dw.assign((size_t)n * (size_t)n, 0.0);
+        const size_t ld = (size_t)dense_ld(n);
+        dw.assign((size_t)n * ld, 0.0);
         for (int64_t c = 0; c < m; ++c) {
-            dw[(size_t)hcu[c] * n + hcv[c]] = J[c];
-            dw[(size_t)hcv[c] * n + hcu[c]] = J[c];
+            dw[(size_t)hcu[c] * ld + hcv[c]] = J[c];
+            dw[(size_t)hcv[c] * ld + hcu[c]] = J[c];
         }
         B200SA_CUDA(cudaMemcpyAsync(base + o.dw, dw.data(), 8 * dw.size(),
                                     cudaMemcpyHostToDevice, plan->stream));
@@ -385,9 +386,9 @@ int b200sa_plan_set_weights_device(b200sa_plan plan, const double *d_h, const do
                 dst.push_back((int64_t)(o.cw / 8) + c);
                 src.push_back((int32_t)(joff + c));
                 if (d.dense) {  // the dense coupling matrix, both triangles
-                    dst.push_back((int64_t)(o.dw / 8) + (int64_t)hcu[c] * d.n + hcv[c]);
+                    dst.push_back((int64_t)(o.dw / 8) + (int64_t)hcu[c] * dense_ld(d.n) + hcv[c]);
                     src.push_back((int32_t)(joff + c));
-                    dst.push_back((int64_t)(o.dw / 8) + (int64_t)hcv[c] * d.n + hcu[c]);
+                    dst.push_back((int64_t)(o.dw / 8) + (int64_t)hcv[c] * dense_ld(d.n) + hcu[c]);
                     src.push_back((int32_t)(joff + c));
                 }
             }
@@ -464,14 +465,16 @@ int b200sa_plan_autotune(b200sa_plan plan, const char *cache_path, int32_t flags
             std::vector<TuneChoice> cands;
             for (int regs = 0; regs < kRegClasses; ++regs)
             for (int stage : {kStageShared, kStageSpins, kStageGlobal, kStageBand}) {
+                const bool dense = (kind & kKindDense) != 0;  // one location and budget
+                if (dense && (stage != kStageShared || regs != dense_reg_class(max_n))) continue;
                 if (stage == kStageShared && max_n > plan->onchip_max) continue;
                 if (stage == kStageBand && (!band_w || (kind & kKindRandom))) continue;
                 const int region =
-                    region_bytes_for_stage(stage, stage == kStageGlobal ? 0 : max_n,
+                    region_bytes_for_stage(stage, stage == kStageGlobal || dense ? 0 : max_n,
                                            stage == kStageBand ? band_w : 0) +
-                    touch_bytes_for((kind & kKindRandom) != 0, max_n);
+                    kind_touch_bytes(kind, max_n);
                 if (region > smem_blk) continue;
-                const int variant = kernel_variant(kind, stage, regs);
+                const int variant = kernel_variant(kind, stage, regs, max_n);
                 int resident[kMaxThreadsPerCta / 32 + 1] = {};
                 int ctas_of[kMaxThreadsPerCta / 32 + 1] = {};
                 int top = 0;

@@ -71,8 +71,9 @@ bool band_allowed() {
     return on;
 }
 
-// Dense updates are on unless the environment sets B200SA_DENSE=0 (results
-// are identical either way; for A/B timing).
+// Small and dense problems keep their state in registers unless the
+// environment sets B200SA_DENSE=0 (results are identical either way; for A/B
+// timing).
 bool dense_allowed() {
     static const bool on = [] {
         const char *e = std::getenv("B200SA_DENSE");
@@ -94,7 +95,7 @@ const uint32_t (*jump_table())[4] {
 
 int occupancy(b200sa_plan_s *P, int variant, int w, int region, int *ctas, char *err,
               size_t errlen) {
-    auto key = std::make_pair((variant << 24) + w, region);
+    auto key = std::make_pair((variant << 8) + w, region);
     auto it = P->occ_cache.find(key);
     if (it != P->occ_cache.end()) {
         *ctas = it->second;
@@ -114,9 +115,10 @@ int shape_for(b200sa_plan_s *P, int kind, int32_t max_n_here, int64_t items, boo
               LaunchShape &out, char *err, size_t errlen, const TuneChoice *choice,
               int band_w_here) {
     const int smem_blk = (int)P->prop.sharedMemPerBlockOptin;
-    const int tb = touch_bytes_for((kind & kKindRandom) != 0, max_n_here);
+    const int tb = kind_touch_bytes(kind, max_n_here);
     if (kind & kKindRandom) band_w_here = 0;  // the band follows a sequential window
     int stage = choice && choice->set ? choice->staging : kStageShared;
+    if (kind & kKindDense) stage = kStageShared;  // (in registers: no other location)
     if (stage == kStageBand &&
         (!band_w_here ||
          region_bytes_for_stage(kStageBand, max_n_here, band_w_here) + tb > smem_blk))
@@ -175,7 +177,7 @@ int shape_for(b200sa_plan_s *P, int kind, int32_t max_n_here, int64_t items, boo
     }
     if (stage == kStageSpins && region_bytes_for_stage(kStageSpins, max_n_here) + tb > smem_blk)
         stage = kStageGlobal;
-    const int cap = stage == kStageGlobal ? 0 : max_n_here;
+    const int cap = stage == kStageGlobal || (kind & kKindDense) ? 0 : max_n_here;
     const int band_cap = stage == kStageBand ? band_w_here : 0;
     const int region = region_bytes_for_stage(stage, cap, band_cap) + tb;
     out.touch_bytes = tb;
@@ -185,10 +187,11 @@ int shape_for(b200sa_plan_s *P, int kind, int32_t max_n_here, int64_t items, boo
     const bool more_warps =
         17 * (region_bytes_for_stage(stage, stage == kStageGlobal ? 0 : max_n_here) + tb) +
             2 * 1024 <= (int)P->prop.sharedMemPerMultiprocessor;
-    const int reg_class = choice && choice->set ? choice->reg_class
+    const int reg_class = (kind & kKindDense)     ? dense_reg_class(max_n_here)
+                          : choice && choice->set ? choice->reg_class
                           : (untuned_global && stage != kStageBand && more_warps) ? 1
                                                                                    : 0;
-    const int variant = kernel_variant(kind, stage, reg_class);
+    const int variant = kernel_variant(kind, stage, reg_class, max_n_here);
     out.stage = stage;
     if (choice && choice->set) {
         // The autotuner's measured configuration (a persistent launch takes
@@ -562,7 +565,6 @@ int b200sa_plan_create(const b200sa_problem *problems, int32_t num_problems,
         o.back = take(8 * n);
         o.bw = take(8 * adj[i].bw.size());
         o.dw = take(8 * adj[i].dense_w.size());
-        o.dbits = take(4 * adj[i].dense_bits.size());
         P->state_off[i + 1] = P->state_off[i] + (int64_t)q.num_reads * q.num_vars;
         P->read_off[i + 1] = P->read_off[i] + q.num_reads;
         P->n.push_back(q.num_vars);
@@ -594,10 +596,8 @@ int b200sa_plan_create(const b200sa_problem *problems, int32_t num_problems,
         }
         if (!adj[i].bw.empty())
             std::memcpy(&staging[o.bw], adj[i].bw.data(), 8 * adj[i].bw.size());
-        if (!adj[i].dense_w.empty()) {
+        if (!adj[i].dense_w.empty())
             std::memcpy(&staging[o.dw], adj[i].dense_w.data(), 8 * adj[i].dense_w.size());
-            std::memcpy(&staging[o.dbits], adj[i].dense_bits.data(), 4 * adj[i].dense_bits.size());
-        }
         if (nb) {
             std::memcpy(&staging[o.betas], q.beta_schedule, 8 * nb);
             double *thr = reinterpret_cast<double *>(&staging[o.thr]);
@@ -644,11 +644,10 @@ int b200sa_plan_create(const b200sa_problem *problems, int32_t num_problems,
                                                  (uint32_t)d.regular_degree
                                            : 0u;
         d.resolve = (adj[i].resolve && resolve_allowed()) ? 1 : 0;
-        d.dense = (d.resolve && adj[i].dense && dense_allowed()) ? 1 : 0;
+        d.dense = (adj[i].dense && dense_allowed()) ? 1 : 0;
         d.back = reinterpret_cast<const uint2 *>(base + o.back);
         d.bw = reinterpret_cast<const double *>(base + o.bw);
         d.dense_w = reinterpret_cast<const double *>(base + o.dw);
-        d.dense_bits = reinterpret_cast<const uint32_t *>(base + o.dbits);
         d.band_b = adj[i].band_b;
         d.band_w = band_allowed() ? adj[i].band_w : 0;
         P->bw_src[i] = std::move(adj[i].bw_src);

@@ -12,13 +12,16 @@
 
 #include "sa_kernel.cuh"
 #include "sa_launch.h"
+#include "sa_dense.cuh"
 #include "sd_kernel.cuh"
 #include "rmc_kernel.cuh"
 #include "pimc_kernel.cuh"
 
 namespace b200sa {
 
-template <bool GIBBS, bool RANDOM_ORDER, bool RESOLVE, int STAGE>
+// K > 0: state in registers, K variables per lane (STAGE is kStageShared, with
+// nothing of the state in the shared region).
+template <bool GIBBS, bool RANDOM_ORDER, bool RESOLVE, int STAGE, int K = 0>
 __device__ __forceinline__ void sa_warp_body(const LaunchArgs &A, int warps_per_cta,
                                              int region_bytes) {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -47,7 +50,7 @@ __device__ __forceinline__ void sa_warp_body(const LaunchArgs &A, int warps_per_
         sp = A.scratch_s + gw * A.scratch_stride;
     }
     if (A.shared_stream && gw != 0) return;
-    if (RANDOM_ORDER) {  // the touch bitmap starts clear; every pass clears what it sets
+    if (RANDOM_ORDER && K == 0) {  // the touch bitmap starts clear; every pass clears what it sets
         for (int i = (int)lane; i < A.touch_bytes / 4; i += 32) touch[i] = 0u;
         __syncwarp();
     }
@@ -84,9 +87,13 @@ __device__ __forceinline__ void sa_warp_body(const LaunchArgs &A, int warps_per_
         const int64_t so = PD->state_offset + (int64_t)r * PD->n;
         WarpCold *cold = warp_cold(ring);
         if (lane == 0) cold->flips = 0ull, cold->passes = 0ull, cold->near = 0u;
-        anneal_read<GIBBS, RANDOM_ORDER, RESOLVE, STAGE>(
-            PD, A.states_in + so, A.states_out + so, &A.energies[rd], de, sp, scratch, ring, rs,
-            lane, touch, band, A.band_cap);
+        if constexpr (K > 0)
+            dense_anneal_read<GIBBS, RANDOM_ORDER, K>(PD, A.states_in + so, A.states_out + so,
+                                                      &A.energies[rd], scratch, ring, rs, lane);
+        else
+            anneal_read<GIBBS, RANDOM_ORDER, RESOLVE, STAGE>(
+                PD, A.states_in + so, A.states_out + so, &A.energies[rd], de, sp, scratch, ring,
+                rs, lane, touch, band, A.band_cap);
         if (lane == 0) {
             A.stats[rd].flips = cold->flips;
             A.stats[rd].passes = cold->passes;
@@ -125,6 +132,13 @@ __global__ void __maxnreg__(kRegs64) sa_warp_kernel_r64(LaunchArgs A, int warps_
     sa_warp_body<GIBBS, RANDOM_ORDER, RESOLVE, STAGE>(A, warps_per_cta, region_bytes);
 }
 
+// State in registers (see dense_reg_class for the budgets).
+template <bool GIBBS, bool RANDOM_ORDER, int K>
+__global__ void __maxnreg__((K <= 2 ? kRegs64 : K <= 4 ? kRegs80 : 128))
+    sa_dense_kernel(LaunchArgs A, int warps_per_cta, int region_bytes) {
+    sa_warp_body<GIBBS, RANDOM_ORDER, false, kStageShared, K>(A, warps_per_cta, region_bytes);
+}
+
 using KernelFn = void (*)(LaunchArgs, int, int);
 
 // Kinds in the order of their numbers (bit 0 Gibbs, bit 1 random order,
@@ -137,17 +151,24 @@ using KernelFn = void (*)(LaunchArgs, int, int);
 #define B200SA_SEQ_KINDS(name, stage)                                                  \
     name<false, false, false, stage>, name<true, false, false, stage>, nullptr, nullptr, \
         name<false, false, true, stage>, name<true, false, true, stage>, nullptr, nullptr
+#define B200SA_DENSE_KINDS(K)                                                          \
+    {sa_dense_kernel<false, false, K>, sa_dense_kernel<true, false, K>,               \
+     sa_dense_kernel<false, true, K>, sa_dense_kernel<true, true, K>}
 #define B200SA_KERNEL_TABLE(name)                                                      \
     {B200SA_KINDS(name, kStageGlobal), B200SA_KINDS(name, kStageShared),              \
      B200SA_KINDS(name, kStageSpins), B200SA_SEQ_KINDS(name, kStageBand)}
 
 static KernelFn kernel_for(int variant) {
-    constexpr int kPerClass = kNumStages * kNumKinds;
+    constexpr int kGeneral = kKindDense;  // kinds below it have a state location
+    constexpr int kPerClass = kNumStages * kGeneral;
     static const KernelFn k128[kPerClass] = B200SA_KERNEL_TABLE(sa_warp_kernel);
     static const KernelFn k80[kPerClass] = B200SA_KERNEL_TABLE(sa_warp_kernel_r80);
     static const KernelFn k64[kPerClass] = B200SA_KERNEL_TABLE(sa_warp_kernel_r64);
-    const int idx = variant & 31;  // kind (bits 0-2) and state location (bits 3-4)
-    if (idx >= kPerClass) return nullptr;
+    static const KernelFn dense[5][4] = {B200SA_DENSE_KINDS(1), B200SA_DENSE_KINDS(2),
+                                         B200SA_DENSE_KINDS(4), B200SA_DENSE_KINDS(8),
+                                         B200SA_DENSE_KINDS(kDenseSlots)};
+    if (variant & kKindDense) return dense[variant >> 8][variant & 3];
+    const int idx = ((variant >> 4) & 3) * kGeneral + (variant & (kGeneral - 1));
     switch (variant_reg_class(variant)) {
         case 0: return k128[idx];
         case 1: return k80[idx];

@@ -16,19 +16,35 @@ constexpr int kRegs64 = 64;
 constexpr int kRegClasses = 3;  // 0: 128, 1: 80, 2: 64
 
 // Kernel kind: bit 0 Gibbs, bit 1 random order, bit 2 in-window resolution
-// (sequential order only; ProblemDev::resolve).
+// (sequential order only; ProblemDev::resolve), bit 3 state in registers
+// (ProblemDev::dense; both orders, without bit 2).
 constexpr int kKindGibbs = 1;
 constexpr int kKindRandom = 2;
 constexpr int kKindResolve = 4;
-constexpr int kNumKinds = 8;
+constexpr int kKindDense = 8;
+constexpr int kNumKinds = 16;
 
-// Kernel variant: bits 0-2 kind, bits 3-4 state location (kStageGlobal,
-// kStageShared, kStageSpins), bits 5-6 register class (0: 128, 1: 80, 2: 64
-// registers).
-inline int kernel_variant(int kind, int stage, int reg_class = 0) {
-    return (kind & (kNumKinds - 1)) | (stage << 3) | (reg_class << 5);
+// Kernels with the state in registers: 1, 2, 4, 8 or kDenseSlots variables per
+// lane by the launch's largest n, one register budget each.
+inline int dense_slots(int max_n) {
+    return max_n <= 32 ? 0 : max_n <= 64 ? 1 : max_n <= 128 ? 2 : max_n <= 256 ? 3 : 4;
 }
-inline int variant_reg_class(int variant) { return variant >> 5; }
+inline int dense_reg_class(int max_n) { return max_n <= 64 ? 2 : max_n <= 128 ? 1 : 0; }
+
+// Kernel variant: bits 0-3 kind, bits 4-5 state location (kStageGlobal,
+// kStageShared, kStageSpins, kStageBand), bits 6-7 register class (0: 128, 1:
+// 80, 2: 64 registers), bits 8-10 dense_slots of kinds with the state in
+// registers.
+inline int kernel_variant(int kind, int stage, int reg_class = 0, int max_n = 0) {
+    return (kind & (kNumKinds - 1)) | (stage << 4) | (reg_class << 6) |
+           ((kind & kKindDense) ? dense_slots(max_n) << 8 : 0);
+}
+inline int variant_reg_class(int variant) { return (variant >> 6) & 3; }
+
+// Bytes of the touch bitmap of a launch (random order outside registers).
+inline int kind_touch_bytes(int kind, int max_n) {
+    return touch_bytes_for((kind & kKindRandom) && !(kind & kKindDense), max_n);
+}
 
 cudaError_t upload_jump_table(const uint32_t table[][4], cudaStream_t stream);
 cudaError_t scatter_weights(double *arena, const int64_t *dst, const int32_t *src, int64_t num_j,

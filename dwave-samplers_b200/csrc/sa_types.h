@@ -4,6 +4,11 @@
 
 #include <vector_types.h>
 
+#ifndef __CUDACC__
+#define __host__
+#define __device__
+#endif
+
 namespace b200sa {
 
 // RNG output ring per read (shared memory).  The ring holds the next
@@ -64,22 +69,23 @@ struct ProblemDev {
     // neighbours, offsets descending (the order the reference adds their
     // flips' contributions).  No list may name a target twice.
     int32_t resolve;
-    // Dense updates (1: on; needs resolve): the committed flips' contributions
-    // are pulled by each variable's owner lane, flip after flip, from
-    // dense_w[j*n + x] (the coupling of j and x) where bit x of
-    // dense_bits[4j ..] is set.  n <= kDenseMaxN.
+    // State in registers (sa_dense.cuh; 1: on): a coupling matrix, row j of
+    // dense_w holding the couplings of variable j (0 where there is none), rows
+    // padded to a multiple of 32, kDenseMaxN readable entries after the last row.
+    // n <= kDenseMaxN, no list names a target twice.
     int32_t dense;
     const uint2 *back;
     const double *bw;
     const double *dense_w;
-    const uint32_t *dense_bits;
     // Banded delta energies (kStageBand): adjacency entries mostly within
     // band_b of their variable; band_w is the shared-memory ring size (a power
     // of two >= 2 band_b + 128), 0 when the problem is not banded.
     int32_t band_b;
     int32_t band_w;
 };
-constexpr int kDenseMaxN = 128;
+constexpr int kDenseSlots = 10;  // variables per lane at most
+constexpr int kDenseMaxN = 32 * kDenseSlots;
+__host__ __device__ inline int dense_ld(int n) { return (n + 31) & ~31; }
 constexpr int kBandMaxSlots = 8192;  // 64 KB of delta energies per warp at most
 
 // Per-read counters written by the kernel.
