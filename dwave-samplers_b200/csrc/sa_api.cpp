@@ -42,7 +42,18 @@ int select_device(int device, cudaDeviceProp &prop, char *err, size_t errlen) {
         return set_err(err, errlen, B200SA_ENODEV,
                        "device index " + std::to_string(device) + " out of range");
     B200SA_CUDA(cudaSetDevice(device));
-    B200SA_CUDA(cudaGetDeviceProperties(&prop, device));
+    {
+        static std::mutex mutex;
+        static std::map<int, cudaDeviceProp> known;
+        std::lock_guard<std::mutex> lock(mutex);
+        auto it = known.find(device);
+        if (it == known.end()) {
+            B200SA_CUDA(cudaGetDeviceProperties(&prop, device));
+            known.emplace(device, prop);
+        } else {
+            prop = it->second;
+        }
+    }
     if (prop.major != 10)
         return set_err(err, errlen, B200SA_ENODEV,
                        std::string("this library is built for sm_100a (B200); device is ") +
@@ -50,6 +61,107 @@ int select_device(int device, cudaDeviceProp &prop, char *err, size_t errlen) {
     return B200SA_OK;
 }
 
+
+namespace {
+
+// What pool_free and pool_stream_free keep, per device.  Never destroyed: the
+// driver takes everything back when the process ends.
+struct DevicePool {
+    std::map<size_t, std::vector<void *>> blocks;  // by size class
+    size_t bytes = 0;
+    std::vector<cudaStream_t> streams;
+};
+std::mutex g_pool_mutex;
+std::map<int, DevicePool> &device_pools() {
+    static auto *pools = new std::map<int, DevicePool>();
+    return *pools;
+}
+
+size_t pool_class(size_t bytes) {
+    size_t c = 512;
+    while (c < bytes) c <<= 1;
+    return c;
+}
+
+}  // namespace
+
+cudaError_t pool_alloc(void **ptr, size_t bytes) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    const size_t size = bytes <= kPoolBlock ? pool_class(bytes) : bytes;
+    if (bytes <= kPoolBlock) {
+        std::lock_guard<std::mutex> lock(g_pool_mutex);
+        DevicePool &pool = device_pools()[device];
+        auto it = pool.blocks.find(size);
+        if (it != pool.blocks.end() && !it->second.empty()) {
+            *ptr = it->second.back();
+            it->second.pop_back();
+            pool.bytes -= size;
+            return cudaSuccess;
+        }
+    }
+    e = cudaMalloc(ptr, size);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    std::vector<void *> back;  // give everything back and try once more
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mutex);
+        DevicePool &pool = device_pools()[device];
+        for (auto &b : pool.blocks) back.insert(back.end(), b.second.begin(), b.second.end());
+        pool.blocks.clear();
+        pool.bytes = 0;
+    }
+    for (void *b : back) cudaFree(b);
+    return cudaMalloc(ptr, bytes <= kPoolBlock ? size : bytes);
+}
+
+void pool_free(void *ptr, size_t bytes, int device) {
+    int current = 0;
+    if (cudaGetDevice(&current) != cudaSuccess) current = device;
+    if (current != device) cudaSetDevice(device);
+    const size_t size = bytes <= kPoolBlock ? pool_class(bytes) : 0;
+    bool kept = false;
+    if (size && cudaDeviceSynchronize() == cudaSuccess) {
+        std::lock_guard<std::mutex> lock(g_pool_mutex);
+        DevicePool &pool = device_pools()[device];
+        if (pool.bytes + size <= kPoolBytes) {
+            pool.blocks[size].push_back(ptr);
+            pool.bytes += size;
+            kept = true;
+        }
+    }
+    if (!kept) cudaFree(ptr);
+    if (current != device) cudaSetDevice(current);
+}
+
+cudaError_t pool_stream(cudaStream_t *stream) {
+    int device = 0;
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mutex);
+        std::vector<cudaStream_t> &free = device_pools()[device].streams;
+        if (!free.empty()) {
+            *stream = free.back();
+            free.pop_back();
+            return cudaSuccess;
+        }
+    }
+    return cudaStreamCreateWithFlags(stream, cudaStreamNonBlocking);
+}
+
+void pool_stream_free(cudaStream_t stream, int device) {
+    if (cudaStreamSynchronize(stream) == cudaSuccess) {
+        std::lock_guard<std::mutex> lock(g_pool_mutex);
+        std::vector<cudaStream_t> &free = device_pools()[device].streams;
+        if (free.size() < kPoolStreams) {
+            free.push_back(stream);
+            return;
+        }
+    }
+    cudaStreamDestroy(stream);
+}
 
 // In-window resolution of the sequential sweep is on unless the environment
 // sets B200SA_RESOLVE=0 (results are identical either way; for A/B timing).
@@ -375,8 +487,8 @@ int collect_stats(b200sa_plan_s *P, const std::vector<std::pair<int, int>> &rang
     return B200SA_OK;
 }
 
-// Persistent mode: one launch per non-empty bucket, spread over forked
-// streams, the bucket with the longest items first so later buckets fill SMs
+// Persistent mode: one launch per non-empty bucket, several of them spread over
+// forked streams, the bucket with the longest items first so later buckets fill SMs
 // as earlier ones drain.
 int run_persistent(b200sa_plan_s *P, LaunchArgs a, cudaStream_t st, char *err,
                    size_t errlen) {
@@ -404,7 +516,7 @@ int run_persistent(b200sa_plan_s *P, LaunchArgs a, cudaStream_t st, char *err,
     }
     if (P->dry_run) return B200SA_OK;
     B200SA_CUDA(cudaMemsetAsync(P->qhead.ptr, 0, sizeof(unsigned long long) * kBuckets, st));
-    B200SA_CUDA(cudaEventRecord(P->fork, st));
+    if (P->streams) B200SA_CUDA(cudaEventRecord(P->fork, st));
     int order[kBuckets];
     for (int b = 0; b < kBuckets; ++b) order[b] = b;
     std::stable_sort(order, order + kBuckets, [&](int x, int y) {
@@ -417,18 +529,22 @@ int run_persistent(b200sa_plan_s *P, LaunchArgs a, cudaStream_t st, char *err,
         const int64_t cnt = P->bucket_off[b + 1] - P->bucket_off[b];
         P->bucket_timed[b] = cnt > 0;
         if (cnt <= 0) continue;
-        const int si = next++ % kStreams;
-        if (!used[si]) B200SA_CUDA(cudaStreamWaitEvent(P->bstream[si], P->fork, 0));
-        used[si] = true;
+        cudaStream_t bs = st;
+        if (P->streams) {
+            const int si = next++ % P->streams;
+            bs = P->bstream[si];
+            if (!used[si]) B200SA_CUDA(cudaStreamWaitEvent(bs, P->fork, 0));
+            used[si] = true;
+        }
         // Inside a capture the timing events become event-record nodes of the
         // graph (external records), so every replay records them.
         const unsigned evflags = P->capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
-        B200SA_CUDA(cudaEventRecordWithFlags(P->bev[b][0], P->bstream[si], evflags));
+        B200SA_CUDA(cudaEventRecordWithFlags(P->bev[b][0], bs, evflags));
         int rc = launch_shape(P, a, shape[b], P->items_lpt.ptr + P->bucket_off[b], cnt,
                               P->bucket_max_n[b], true, false, P->qhead.ptr + b, slot0[b],
-                              P->bstream[si], err, errlen);
+                              bs, err, errlen);
         if (rc) return rc;
-        B200SA_CUDA(cudaEventRecordWithFlags(P->bev[b][1], P->bstream[si], evflags));
+        B200SA_CUDA(cudaEventRecordWithFlags(P->bev[b][1], bs, evflags));
         P->bshape[b] = shape[b];
     }
     for (int si = 0; si < kStreams; ++si) {
@@ -482,16 +598,9 @@ int b200sa_plan_create(const b200sa_problem *problems, int32_t num_problems,
     int rc = select_device(device, P->prop, err, errlen);
     if (rc) return rc;
     P->device = device;
-    B200SA_CUDA(cudaStreamCreateWithFlags(&P->stream, cudaStreamNonBlocking));
-    for (int b = 0; b < kStreams; ++b) {
-        B200SA_CUDA(cudaStreamCreateWithFlags(&P->bstream[b], cudaStreamNonBlocking));
-        B200SA_CUDA(cudaEventCreateWithFlags(&P->join[b], cudaEventDisableTiming));
-    }
+    B200SA_CUDA(pool_stream(&P->stream));
     B200SA_CUDA(cudaEventCreate(&P->ev0));
     B200SA_CUDA(cudaEventCreate(&P->ev1));
-    B200SA_CUDA(cudaEventCreateWithFlags(&P->fork, cudaEventDisableTiming));
-    for (int b = 0; b < kBuckets; ++b)
-        for (int k = 0; k < 2; ++k) B200SA_CUDA(cudaEventCreate(&P->bev[b][k]));
     P->num_problems = num_problems;
     // On chip when at least three warps' regions fit in one SM.
     {
@@ -695,6 +804,21 @@ int b200sa_plan_create(const b200sa_problem *problems, int32_t num_problems,
         P->bucket_off[b + 1]++;
         P->bucket_max_n[b] = std::max(P->bucket_max_n[b], P->n[p]);
         P->bucket_lead_cost[b] = std::max(P->bucket_lead_cost[b], cost(it));
+    }
+    {
+        int used = 0;
+        for (int b = 0; b < kBuckets; ++b) {
+            if (P->bucket_off[b + 1] == 0) continue;  // (still counts)
+            ++used;
+            for (int k = 0; k < 2; ++k) B200SA_CUDA(cudaEventCreate(&P->bev[b][k]));
+        }
+        P->streams = used > 1 ? std::min(used, kStreams) : 0;
+        if (P->streams)
+            B200SA_CUDA(cudaEventCreateWithFlags(&P->fork, cudaEventDisableTiming));
+        for (int si = 0; si < P->streams; ++si) {
+            B200SA_CUDA(pool_stream(&P->bstream[si]));
+            B200SA_CUDA(cudaEventCreateWithFlags(&P->join[si], cudaEventDisableTiming));
+        }
     }
     for (int b = 0; b < kBuckets; ++b) P->bucket_off[b + 1] += P->bucket_off[b];
     // A bucket may use the band location when all of its problems are banded.
