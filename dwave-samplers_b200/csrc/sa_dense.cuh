@@ -26,54 +26,6 @@
 
 namespace b200sa {
 
-// log2 of a draw for the acceptance bounds, from its upper half: truncation
-// and rounding stay below 2^-18 for draws of 2^52 and more; smaller ones
-// (2^-12 of all) give NaN, which leaves the decision to the exact test.
-__device__ __forceinline__ float draw_log2(uint64_t r) {
-    const uint32_t hi = (uint32_t)(r >> 32);
-    const float y = lg2_approx(__uint2float_rn(hi)) + 32.0f;
-    return hi >= (1u << 20) ? y : __int_as_float(0x7fffffff);
-}
-
-// A lane's decision on its delta energy d (cpu_sa.cpp:140-166): whether it
-// draws, and the bound t that the log2 of an accepted draw stays below (see
-// metropolis_fast and gibbs_fast): +inf for a flip without a draw, -inf for
-// none.  The bound is taken from d in single precision, which adds two roundings
-// of a product below 64; betas beyond the range of that give NaN, which leaves
-// every decision to the exact test.
-template <bool GIBBS>
-struct DenseChoice {
-    bool need;
-    float t;
-
-    // Per beta: beta log2(e), the factor of d.
-    static __device__ __forceinline__ float scale(double beta) {
-        return beta > 1e-30 && beta < 1e30 ? (float)(beta * (double)kLog2e)
-                                           : __int_as_float(0x7fffffff);
-    }
-    __device__ __forceinline__ void look(double d, float scale, double thr, bool act) {
-        const float inf = __int_as_float(0x7f800000);
-        const bool cons = act && !(d >= thr);
-        const float z = (float)d * scale;  // log2(exp(d * beta))
-        if constexpr (GIBBS) {
-            need = cons;
-            // log2(1 + exp(z)), see gibbs_fast
-            const float big = 24.0f * kLog2e;
-            const float g = z > big ? z : z < -big ? 0.0f : lg2_approx(1.0f + ex2_approx(z));
-            t = cons ? 64.0f - g : -inf;
-        } else {
-            const bool down = d <= 0.0;
-            need = cons && !down;
-            t = !cons ? -inf : down ? inf : 64.0f - z;
-        }
-    }
-    // The exact decision.  Bit 0: flips, bit 1: near tie.
-    __device__ __forceinline__ int exact(double d, double beta, uint64_t r) const {
-        if (!need) return t > 0.0f ? 1 : 0;
-        return GIBBS ? gibbs_exact(d, beta, r) : metropolis_exact(d, beta, r);
-    }
-};
-
 // The state of one read.  PM1: every spin is +1 or -1, kept as a sign bit; a
 // contribution ((int8)(4 s_j) J) s_x is then J times +4 or -4, exactly.
 template <bool PM1, int K>
@@ -145,7 +97,7 @@ __device__ __forceinline__ void dense_sweep_sequential(DenseState<PM1, K> &S, in
     using Spin = typename State::Spin;
     const unsigned lt_mask = (1u << lane) - 1u;
     const float inf = __int_as_float(0x7f800000);
-    const float scale = DenseChoice<GIBBS>::scale(beta);
+    const float scale = Choice<GIBBS>::scale(beta);
     // (Unrolled only while the copies of the body stay small.)
 #pragma unroll(K <= 4 ? K : 1)
     for (int w = 0; w < K; ++w) {
@@ -157,7 +109,7 @@ __device__ __forceinline__ void dense_sweep_sequential(DenseState<PM1, K> &S, in
 #pragma unroll
         for (int i = 0; i < K; ++i)
             if (i == w) d = S.d[i], s = S.spin(i);
-        DenseChoice<GIBBS> ch;
+        Choice<GIBBS> ch;
         ch.look(d, scale, thr, act);
         unsigned nm = __ballot_sync(kFull, ch.need);
         unsigned flips = 0u, ties = 0u;
@@ -200,7 +152,7 @@ __device__ __forceinline__ void dense_sweep_sequential(DenseState<PM1, K> &S, in
                 if (!again) break;
                 // A tie of a lane that decides anew is no longer one.
                 ties &= (1u << (c - 1)) | ((1u << (c - 1)) - 1u);
-                DenseChoice<GIBBS> next;
+                Choice<GIBBS> next;
                 next.look(d, scale, thr, act);
                 const bool mine = (int)lane >= c;
                 ch.t = mine ? next.t : -inf;  // committed lanes decide no more
@@ -228,7 +180,7 @@ __device__ __forceinline__ void dense_sweep_random(DenseState<PM1, K> &S, int n,
     using State = DenseState<PM1, K>;
     using Spin = typename State::Spin;
     const double *matrix = S.w - lane;
-    const float scale = DenseChoice<GIBBS>::scale(beta);
+    const float scale = Choice<GIBBS>::scale(beta);
     for (int rem = n; rem > 0;) {
         ring_refill(ring, rs, lane);
         const int var = mod_n(ring[(rs.q + lane) & (kRing - 1)], (uint32_t)n, magic);
@@ -241,7 +193,7 @@ __device__ __forceinline__ void dense_sweep_random(DenseState<PM1, K> &S, int n,
             const Spin si = __shfl_sync(kFull, S.spin(i), var & 31);
             if (var >> 5 == i) d = di, s = si;
         }
-        DenseChoice<GIBBS> ch;
+        Choice<GIBBS> ch;
         ch.look(d, scale, thr, true);
         unsigned flips = 0u, ties = 0u, live = kFull, C, N;
         for (;;) {
@@ -297,7 +249,7 @@ __device__ __forceinline__ void dense_sweep_random(DenseState<PM1, K> &S, int n,
             }
             if (!again) break;
             ties &= ~live;
-            DenseChoice<GIBBS> next;
+            Choice<GIBBS> next;
             next.look(d, scale, thr, true);
             if ((live >> lane) & 1u) ch = next;
         }

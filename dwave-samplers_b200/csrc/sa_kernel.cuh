@@ -679,32 +679,63 @@ __device__ __forceinline__ int decide(double d, double beta, uint64_t r) {
     return GIBBS ? gibbs_exact(d, beta, r) : metropolis_exact(d, beta, r);
 }
 
+// log2 of a draw for the acceptance bounds, from its upper half: truncation
+// and rounding stay below 2^-18 for draws of 2^52 and more; smaller ones
+// (2^-12 of all) give NaN, which leaves the decision to the exact test.
+__device__ __forceinline__ float draw_log2(uint64_t r) {
+    const uint32_t hi = (uint32_t)(r >> 32);
+    const float y = lg2_approx(__uint2float_rn(hi)) + 32.0f;
+    return hi >= (1u << 20) ? y : __int_as_float(0x7fffffff);
+}
+
+// A lane's decision on its delta energy d (cpu_sa.cpp:140-166): whether it
+// draws, and the bound t that the log2 of an accepted draw stays below (see
+// metropolis_fast and gibbs_fast): +inf for a flip without a draw, -inf for
+// none.  The bound is taken from d in single precision, which adds two roundings
+// of a product below 64; betas beyond the range of that give NaN, which leaves
+// every decision to the exact test.
+template <bool GIBBS>
+struct Choice {
+    bool need;
+    float t;
+
+    // Per beta: beta log2(e), the factor of d.
+    static __device__ __forceinline__ float scale(double beta) {
+        return beta > 1e-30 && beta < 1e30 ? (float)(beta * (double)kLog2e)
+                                           : __int_as_float(0x7fffffff);
+    }
+    __device__ __forceinline__ void look(double d, float scale, double thr, bool act) {
+        const float inf = __int_as_float(0x7f800000);
+        const bool cons = act && !(d >= thr);
+        const float z = (float)d * scale;  // log2(exp(d * beta))
+        if constexpr (GIBBS) {
+            need = cons;
+            // log2(1 + exp(z)), see gibbs_fast
+            const float big = 24.0f * kLog2e;
+            const float g = z > big ? z : z < -big ? 0.0f : lg2_approx(1.0f + ex2_approx(z));
+            t = cons ? 64.0f - g : -inf;
+        } else {
+            const bool down = d <= 0.0;
+            need = cons && !down;
+            t = !cons ? -inf : down ? inf : 64.0f - z;
+        }
+    }
+    // The exact decision.  Bit 0: flips, bit 1: near tie.
+    __device__ __forceinline__ int exact(double d, double beta, uint64_t r) const {
+        if (!need) return t > 0.0f ? 1 : 0;
+        return GIBBS ? gibbs_exact(d, beta, r) : metropolis_exact(d, beta, r);
+    }
+};
+
 // Sequential order (cpu_sa.cpp:132-192) in speculative passes over windows
 // of 32 consecutive variables, one per lane.  Every lane decides its variable
-// against the delta energies at the start of the pass; the first round
-// commits the prefix of the window that ends before the first variable whose
-// decision a committed flip could have changed (a later neighbour of an
-// accepted flip), so the committed decisions equal the sequential ones.
-//
-// With `resolve` (problems whose lists name no target twice, reads whose
-// spins are all +-1) the pass goes on in further rounds instead of ending
-// there.  The flips committed by a round add their contributions
-// ((4 s_j) J) s_k (cpu_sa.cpp:172-185) to the delta energies, held in
-// registers, of the uncommitted lanes they neighbour, in variable order as the
-// reference adds them; those lanes decide again, their draws placed after the
-// ones already committed, and the next commit point follows by the same rule.
-// Each round commits at least its first lane.  The update phase then applies
-// every committed flip's entries to the delta energies in memory in entry
-// order with the spins as they were at the start of the pass, and negates the
-// flipped variables' own delta energies last: negation is exact and commutes
-// with rounding, so a contribution added after the negation in the reference
-// (a neighbour that flipped earlier) equals the negated contribution added
-// before it.
+// against the delta energies at the start of the pass; the pass commits the
+// prefix of the window that ends before the first variable whose decision a
+// committed flip could have changed (a later neighbour of an accepted flip),
+// so the committed decisions equal the sequential ones.
 //
 // While a window is processed, the records of the next one are prefetched
-// into L1 when the delta energies are on chip or in the band; with resolution
-// also the lines of this window's adjacency lists, which the update phase
-// reads.
+// into L1 when the delta energies are on chip or in the band.
 //
 // BANDED (kStageBand): the delta energies of variables within band_b of the
 // window live in a shared-memory ring of band_w slots (BandDe), the rest in
@@ -716,12 +747,49 @@ __device__ __forceinline__ int decide(double d, double beta, uint64_t r) {
 // decisions read the window; an update through a coupler longer than band_b
 // can reach the last slide's slots, so the update phase waits for all of
 // them.  At every sweep the band is written back and reloaded from the start.
+//
+// The band at the start of a sweep: written back (when `live`) and reloaded
+// around variable 0.
+__device__ __forceinline__ void band_rewind(BandDe &de, int n, int band_b, bool live,
+                                            unsigned lane) {
+    cp_async_wait<0>();
+    __syncwarp();
+    const int w = (int)de.w;
+    const unsigned mask = de.w - 1u;
+    if (live) {
+        for (int i = (int)lane; i < w; i += 32) {
+            const int x = de.lo + i;
+            if (x >= 0 && x < n) de.g[x] = de.b[(unsigned)x & mask];
+        }
+        __syncwarp();
+    }
+    de.lo = -band_b;
+    const int top = min(n, w - band_b);
+    for (int x = (int)lane; x < top; x += 32) de.b[(unsigned)x & mask] = de.g[x];
+    __syncwarp();
+}
+
+// The band after a pass over the window at p that committed c variables.
+__device__ __forceinline__ void band_slide(const BandDe &de, int n, int p, int band_b, int c,
+                                           unsigned lane) {
+    __syncwarp();
+    if ((int)lane < c) {
+        const int xo = p - band_b + (int)lane;  // < p: band_b >= 32
+        const unsigned slot = (unsigned)xo & (de.w - 1u);
+        if (xo >= 0) de.g[xo] = de.b[slot];
+        const int xn = xo + (int)de.w;
+        if (xn < n) cp_async8(&de.b[slot], &de.g[xn]);
+    }
+    cp_async_commit();
+    __syncwarp();
+}
+
 template <bool GIBBS, int STAGE>
 __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
                                                  int8_t *sp, double *scratch,
                                                  uint64_t *ring, RingState &rs,
-                                                 unsigned lane, bool resolve,
-                                                 double *band, int band_w, int band_b) {
+                                                 unsigned lane, double *band, int band_w,
+                                                 int band_b) {
     constexpr bool BANDED = STAGE == kStageBand;
     const int n = P.n;
     const int D = P.regular_degree;
@@ -739,23 +807,8 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
         for (int sw = 0; sw < reload(P.pd->sweeps_per_beta); ++sw) {
             SweepCount cnt;
             if constexpr (BANDED) {
-                if (band_w) {  // write the band back, reload it at the start
-                    cp_async_wait<0>();
-                    __syncwarp();
-                    const unsigned mask = (unsigned)band_w - 1u;
-                    if (band_live) {
-                        for (int i = (int)lane; i < band_w; i += 32) {
-                            const int x = de.lo + i;
-                            if (x >= 0 && x < n) de_g[x] = band[(unsigned)x & mask];
-                        }
-                        __syncwarp();
-                    }
-                    de.lo = -band_b;
-                    const int top = min(n, band_w - band_b);
-                    for (int x = (int)lane; x < top; x += 32) band[(unsigned)x & mask] = de_g[x];
-                    __syncwarp();
-                    band_live = true;
-                }
+                if (band_w) band_rewind(de, n, band_b, band_live, lane);
+                band_live = true;
             }
             int p = 0;
             while (p < n) {
@@ -773,23 +826,13 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
                 int dist = (int)kDistCap;
                 uint32_t shr = 0u;
                 uint2 vi = make_uint2(0u, 0u);
-                uint2 bk = make_uint2(0u, 0u);
                 int s_cur = 0;
                 if (act) {
                     d = de.get(v);
                     dist = __ldg(&P.dist[v]);
                     shr = __ldg(&P.share[v]);
                     if (!D) vi = __ldg(&P.vinfo[v]);
-                    if (resolve) bk = __ldg(&P.back[v]);
                     s_cur = (int)sp[v];
-                }
-                // The nearest back neighbour's coupling (stored last), loaded
-                // ahead: on lattices and chains it is the one the rounds need.
-                int o_near = 0;
-                double bw_near = 0.0;
-                if (resolve && bk.x) {
-                    o_near = __ffs(bk.x) - 1;
-                    bw_near = __ldg(&P.bw[bk.y + (uint32_t)__popc(bk.x) - 1u]);
                 }
                 if (act) {
                     // The next window starts at p + c <= p + 32 and ends
@@ -802,12 +845,6 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
                         prefetch_l1(P.dist + vn);
                         prefetch_l1(P.share + vn);
                         if (!D) prefetch_l1(P.vinfo + vn);
-                        if (resolve) prefetch_l1(P.back + vn);
-                    }
-                    if (resolve) {  // the update phase's lists (no early load with resolution)
-                        const uint32_t e0 = D ? (uint32_t)v * (uint32_t)D : vi.x;
-                        prefetch_l1(P.col + e0);
-                        prefetch_l1(P.w + e0);
                     }
                 }
                 const bool consider = act && !(d >= thr);  // cpu_sa.cpp:140
@@ -823,14 +860,12 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
                 }
                 const unsigned am = __ballot_sync(kFull, acc);
                 // Equal-length lists: start loading the accepted flips'
-                // adjacency before the commit point is known (not with
-                // resolution, whose later rounds change the accepted set).
-                const bool pre = !resolve;
+                // adjacency before the commit point is known.
                 const double mult = (double)(int)(int8_t)(4 * s_cur);
                 PreEntries pe;
 #pragma unroll
                 for (int i = 0; i < kPreGroups; ++i) pe.nb[i] = 0, pe.k[i] = 0, pe.w[i] = 0.0;
-                if (D && am && pre) {
+                if (D && am) {
                     if (acc) rank_tab[__popc(am & lt_mask)] = (int)lane;
                     __syncwarp();
                     const int pre_n = min(__popc(am) * D, 32 * kPreGroups);
@@ -841,64 +876,11 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
                     }
                 }
                 const int bound = acc ? (int)lane + dist : 32;
-                int c = min(__reduce_min_sync(kFull, bound), L);
-                unsigned done = c >= 32 ? kFull : ((1u << c) - 1u);
-                uint32_t used = (uint32_t)__popc(nm & done);
-                unsigned fm = am & done;
-                unsigned nearm = __ballot_sync(kFull, near) & done;
-                if (resolve && c < L) {
-                    // Lanes j < lane whose variables neighbour this lane's.
-                    const unsigned back_lanes = __brev(bk.x) >> (31u - lane);
-                    const unsigned smask = __ballot_sync(kFull, s_cur > 0);
-                    const double sk = (double)s_cur;
-                    unsigned newf = fm;
-                    // Each lane keeps the flags of its latest decision; a
-                    // committed lane's are final, so the ballots of a round
-                    // cover the committed lanes too (its draw position counts
-                    // the committed draws before it).
-                    bool need_l = need, acc_l = acc;
-                    unsigned nm_all;
-                    do {
-                        const bool live = act && (int)lane >= c;
-                        unsigned rel = live ? back_lanes & newf : 0u;
-                        while (rel) {
-                            const int j = __ffs(rel) - 1;
-                            rel &= rel - 1u;
-                            const int o = (int)lane - j;
-                            double wj = bw_near;
-                            if (o != o_near) {
-                                // Offsets are stored descending: o's rank is
-                                // the number of larger offsets.
-                                wj = __ldg(&P.bw[bk.y + (uint32_t)__popc((bk.x >> o) >> 1)]);
-                            }
-                            const double mj = ((smask >> j) & 1u) ? 4.0 : -4.0;
-                            d = __dadd_rn(d, __dmul_rn(__dmul_rn(mj, wj), sk));
-                        }
-                        if (live) {
-                            const bool cons2 = !(d >= thr);
-                            need_l = GIBBS ? cons2 : (cons2 && !(d <= 0.0));
-                            acc_l = GIBBS ? false : cons2;
-                            near = false;
-                        }
-                        nm_all = __ballot_sync(kFull, need_l);
-                        if (live && need_l) {
-                            const uint64_t r =
-                                ring[(rs.q + (uint32_t)__popc(nm_all & lt_mask)) & (kRing - 1)];
-                            const int x = decide<GIBBS>(d, beta, r);
-                            acc_l = (x & 1) != 0;
-                            near = (x & 2) != 0;
-                        }
-                        const unsigned am_all = __ballot_sync(kFull, acc_l);
-                        const int bound2 = (live && acc_l) ? (int)lane + dist : 32;
-                        c = min(__reduce_min_sync(kFull, bound2), L);
-                        const unsigned upto = c >= 32 ? kFull : ((1u << c) - 1u);
-                        newf = am_all & upto & ~done;
-                        fm = am_all & upto;
-                        done = upto;
-                    } while (c < L);
-                    used = (uint32_t)__popc(nm_all & done);
-                    nearm = __ballot_sync(kFull, near) & done;
-                }
+                const int c = min(__reduce_min_sync(kFull, bound), L);
+                const unsigned done = c >= 32 ? kFull : ((1u << c) - 1u);
+                const uint32_t used = (uint32_t)__popc(nm & done);
+                const unsigned fm = am & done;
+                const unsigned nearm = __ballot_sync(kFull, near) & done;
                 rs.q += used;
                 cnt.pass((unsigned)__popc(fm), (unsigned)__popc(nearm));
                 if constexpr (BANDED) {
@@ -917,18 +899,14 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
                     const bool f = (fm >> lane) & 1u;
                     const bool may_conflict =
                         __any_sync(kFull, f && ((shr & 1u) || ((shr >> 1) & later)));
-                    // Without resolution the committed flips are pairwise
-                    // non-adjacent, so a flip's own slot receives an addition
-                    // in this pass only from a repeated target in its own
-                    // list; otherwise it still holds the window value d and
-                    // the negation needs no load.
-                    const bool own_fresh = !resolve && !(shr & 1u);
+                    // The committed flips are pairwise non-adjacent, so a
+                    // flip's own slot receives an addition in this pass only
+                    // from a repeated target in its own list; otherwise it
+                    // still holds the window value d and the negation needs no
+                    // load.
+                    const bool own_fresh = !(shr & 1u);
                     if (D) {
-                        if (!pre) {
-                            if (f) rank_tab[__popc(fm & lt_mask)] = (int)lane;
-                            __syncwarp();
-                        }
-                        update_regular(P, de, sp, scratch, rank_tab, __popc(fm), p, pre, pe,
+                        update_regular(P, de, sp, scratch, rank_tab, __popc(fm), p, true, pe,
                                        may_conflict, mult, lane);
                         if (f) {  // cpu_sa.cpp:189-190, after the variable's own updates
                             sp[v] = (int8_t)(-s_cur);
@@ -942,21 +920,214 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
                     }
                 }
                 if constexpr (BANDED) {
-                    if (band_w) {  // slide the band by c
-                        __syncwarp();
-                        if ((int)lane < c) {
-                            const int xo = p - band_b + (int)lane;  // < p: band_b >= 32
-                            const unsigned slot = (unsigned)xo & ((unsigned)band_w - 1u);
-                            if (xo >= 0) de_g[xo] = band[slot];
-                            const int xn = xo + band_w;
-                            if (xn < n) cp_async8(&band[slot], &de_g[xn]);
-                        }
-                        cp_async_commit();
-                        __syncwarp();
-                    }
+                    if (band_w) band_slide(de, n, p, band_b, c, lane);
                 }
                 p += c;
                 if constexpr (BANDED) de.lo = p - band_b;
+            }
+            cnt.flush(ring, lane);
+        }
+    }
+    if constexpr (BANDED) {
+        if (band_w) {  // nothing of this read may land after it
+            cp_async_wait<0>();
+            __syncwarp();
+        }
+    }
+}
+
+// Sequential order for problems whose window variables often neighbour each
+// other (`resolve`: lists name no target twice), on reads whose spins are all
+// +-1.  Every pass commits its whole window.
+//
+// The decisions of a window solve a recursion: lane k's delta energy is the one
+// at the start of the pass plus ((4 s_j) J) s_k of every flipped lane j < k it
+// neighbours, in variable order (cpu_sa.cpp:172-185), and its draw is placed
+// after those of the drawing lanes before it.  The lanes solve it together:
+// from an assumed set of flips all of them decide at once, the flips that come
+// out are the next assumption, until a set reproduces itself.  A lane's
+// decision depends on earlier lanes only, so after i rounds at least the first
+// i lanes are as in the reference, and the set that reproduces itself is the
+// reference's.  Changes die out quickly, so rounds are few.  (Committing up to
+// the first dependent lane per round and deciding the rest anew took about one
+// round per dependent flip: L = 32 lattice, 256 reads x 64 sweeps 226 -> 171 ms;
+// L = 8, 4096 x 50 5.0 -> 3.4; L = 16, 1000 x 20 11.9 -> 7.4.)
+//
+// The update phase then applies every flip's entries to the delta energies in
+// memory in entry order with the spins as they were at the start of the pass,
+// and negates the flipped variables' own delta energies last: negation is
+// exact and commutes with rounding, so a contribution added after the negation
+// in the reference (a neighbour that flipped earlier) equals the negated
+// contribution added before it.
+//
+// Delta energies on chip or in the band: the next window's records are loaded
+// into registers while this one is worked on (a window always starts 32
+// further on), its lists brought into L1.
+template <bool GIBBS, int STAGE>
+__device__ __forceinline__ void sweep_resolved(const Prob &P, double *de_g, int8_t *sp,
+                                               double *scratch, uint64_t *ring, RingState &rs,
+                                               unsigned lane, double *band, int band_w,
+                                               int band_b) {
+    constexpr bool BANDED = STAGE == kStageBand;
+    constexpr bool AHEAD = !DeFor<STAGE>::T::kAsyncAdd;
+    const int n = P.n;
+    const int D = P.regular_degree;
+    const unsigned lt_mask = (1u << lane) - 1u;
+    const float inf = __int_as_float(0x7f800000);
+    int *rank_tab = reinterpret_cast<int *>(scratch + 32);
+    typename DeFor<STAGE>::T de;
+    bool band_live = false;
+    if constexpr (BANDED)
+        de = BandDe{de_g, band, 0, (unsigned)band_w};
+    else
+        de.p = de_g;
+    // A variable's records.  `near` is the coupling of the nearest back
+    // neighbour (stored last), on lattices and chains the one that matters.
+    struct Record {
+        uint32_t shr;
+        uint2 vi, bk;
+        double near;
+    };
+    auto load = [&](int v) {
+        Record r{0u, make_uint2(0u, 0u), make_uint2(0u, 0u), 0.0};
+        if (v < n) {
+            r.shr = __ldg(&P.share[v]);
+            r.vi = D ? make_uint2((uint32_t)v * (uint32_t)D, (uint32_t)D) : __ldg(&P.vinfo[v]);
+            r.bk = __ldg(&P.back[v]);
+        }
+        return r;
+    };
+    auto load_near = [&](Record &r) {
+        if (r.bk.x) r.near = __ldg(&P.bw[r.bk.y + (uint32_t)__popc(r.bk.x) - 1u]);
+    };
+    Record next = load((int)lane);
+    load_near(next);
+    for (int b = 0; b < reload(P.pd->num_betas); ++b) {
+        const double beta = __ldg(&reload(P.pd->betas)[b]);
+        const double thr = __ldg(&reload(P.pd->thresholds)[b]);
+        const float scale = Choice<GIBBS>::scale(beta);
+        for (int sw = 0; sw < reload(P.pd->sweeps_per_beta); ++sw) {
+            SweepCount cnt;
+            if constexpr (BANDED) {
+                if (band_w) band_rewind(de, n, band_b, band_live, lane);
+                band_live = true;
+            }
+            for (int p = 0; p < n; p += 32) {
+                if constexpr (BANDED) {
+                    if (band_w) {  // the slides of all but the last pass have landed
+                        cp_async_wait<1>();
+                        __syncwarp();
+                    }
+                }
+                ring_refill(ring, rs, lane);
+                const int v = p + (int)lane;
+                const bool act = v < n;
+                double d0 = 0.0;
+                int s_cur = 0;
+                if (act) {
+                    d0 = de.get(v);
+                    s_cur = (int)sp[v];
+                }
+                Record r;
+                if constexpr (AHEAD) {
+                    r = next;
+                    const int vn = p + 32 < n ? v + 32 : (int)lane;
+                    next = load(vn);
+                    const uint32_t e0 = D ? next.vi.x : r.vi.x;
+                    if ((D ? vn : v) < n) {
+                        prefetch_l1(P.col + e0);
+                        prefetch_l1(P.w + e0);
+                    }
+                } else {
+                    r = load(v);
+                    load_near(r);
+                }
+                double d = d0;
+                Choice<GIBBS> ch;
+                ch.look(d, scale, thr, act);
+                unsigned fm = 0u, ties = 0u;
+                // (A bound of NaN counts as a decision to be made.)
+                if (__any_sync(kFull, !(ch.t == -inf))) {
+                    const float y = draw_log2(ring[(rs.q + lane) & (kRing - 1)]);
+                    // Lanes before this one whose variables neighbour its own.
+                    const unsigned back = act ? __brev(r.bk.x) >> (31u - lane) : 0u;
+                    const int o_near = r.bk.x ? __ffs(r.bk.x) - 1 : 0;
+                    const unsigned up = __ballot_sync(kFull, s_cur > 0);
+                    unsigned rel = 0u;  // flipped lanes among `back`, as d holds them
+                    unsigned nm;
+                    for (;;) {
+                        nm = __ballot_sync(kFull, ch.need);
+                        const int at = __popc(nm & lt_mask);
+                        const float gap = ch.t - __shfl_sync(kFull, y, at);
+                        fm = __ballot_sync(kFull, gap > kBand);
+                        ties = 0u;
+                        if (__any_sync(kFull, !(fabsf(gap) > kBand))) {  // inside the band
+                            int x = 0;
+                            if (!(fabsf(gap) > kBand))
+                                x = ch.exact(d, beta, ring[(rs.q + (uint32_t)at) & (kRing - 1)]);
+                            fm |= __ballot_sync(kFull, (x & 1) != 0);
+                            ties = __ballot_sync(kFull, (x & 2) != 0);
+                        }
+                        const bool changed = (back & fm) != rel;
+                        if (!__any_sync(kFull, changed)) break;
+                        if (changed) {
+                            rel = back & fm;
+                            d = d0;
+                            for (unsigned m = rel; m; m &= m - 1u) {
+                                const int j = __ffs(m) - 1;
+                                const int o = (int)lane - j;
+                                double wj = r.near;
+                                if (o != o_near)  // offsets are stored descending
+                                    wj = __ldg(&P.bw[r.bk.y +
+                                                     (uint32_t)__popc((r.bk.x >> o) >> 1)]);
+                                // ((4 s_j) J) s_k, exactly +-4 J
+                                const bool same = (((up >> j) & 1u) != 0u) == (s_cur > 0);
+                                d = __dadd_rn(d, __dmul_rn(wj, same ? 4.0 : -4.0));
+                            }
+                            ch.look(d, scale, thr, act);
+                        }
+                    }
+                    rs.q += (uint32_t)__popc(nm);
+                }
+                cnt.pass((unsigned)__popc(fm), (unsigned)__popc(ties));
+                if (fm) {
+                    if constexpr (BANDED) {
+                        // The slots the last slide fetched lie at the far end
+                        // of the band, which only an update through a coupler
+                        // longer than band_b can reach: they land before the
+                        // update phase.
+                        if (band_w) {
+                            cp_async_wait<0>();
+                            __syncwarp();
+                        }
+                    }
+                    // A slot can receive two additions only through a
+                    // neighbour common to two flips.
+                    const unsigned later = lane < 31 ? fm >> (lane + 1) : 0u;
+                    const bool f = (fm >> lane) & 1u;
+                    const bool may_conflict = __any_sync(kFull, f && ((r.shr >> 1) & later));
+                    if (D) {
+                        if (f) rank_tab[__popc(fm & lt_mask)] = (int)lane;
+                        __syncwarp();
+                        const PreEntries none{};
+                        update_regular(P, de, sp, scratch, rank_tab, __popc(fm), p, false, none,
+                                       may_conflict, (double)(4 * s_cur), lane);
+                        if (f) {  // cpu_sa.cpp:189-190, after the variable's own updates
+                            sp[v] = (int8_t)(-s_cur);
+                            de.set(v, -de.get(v));
+                        }
+                        __syncwarp();
+                    } else {
+                        apply_flips(P, de, sp, scratch, fm, v, (int)r.vi.x,
+                                    (int)(r.vi.y & kDegMask), s_cur, may_conflict, lane);
+                    }
+                }
+                if constexpr (BANDED) {
+                    const int c = min(32, n - p);
+                    if (band_w) band_slide(de, n, p, band_b, c, lane);
+                    de.lo = p + c - band_b;
+                }
+                if constexpr (AHEAD) load_near(next);
             }
             cnt.flush(ring, lane);
         }
@@ -1189,8 +1360,12 @@ __device__ __forceinline__ void anneal_read(const ProblemDev *PD, const int8_t *
             const int bw = (STAGE == kStageBand && PD->band_w > 0 && PD->band_w <= band_cap)
                                ? PD->band_w
                                : 0;
-            sweep_sequential<GIBBS, STAGE>(P, de, sp, scratch, ring, rs, lane,
-                                                    RESOLVE && pm1, band, bw, PD->band_b);
+            if (RESOLVE && pm1)
+                sweep_resolved<GIBBS, STAGE>(P, de, sp, scratch, ring, rs, lane, band, bw,
+                                             PD->band_b);
+            else
+                sweep_sequential<GIBBS, STAGE>(P, de, sp, scratch, ring, rs, lane, band, bw,
+                                               PD->band_b);
         }
     }
     __syncwarp();
