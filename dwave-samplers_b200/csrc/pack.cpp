@@ -91,6 +91,7 @@ void pack_adjacency(const b200sa_problem &p, PackedAdjacency &out) {
     // Speculation record: nearest later neighbour; repeated targets; pairs
     // of variables less than 32 apart with a common neighbour.
     out.share.assign((size_t)n, 0u);
+    out.wshare.assign((size_t)n, 0u);
     out.dist.assign((size_t)n, 0u);
     {
         std::vector<int32_t> nb;
@@ -99,8 +100,14 @@ void pack_adjacency(const b200sa_problem &p, PackedAdjacency &out) {
             std::sort(nb.begin(), nb.end());
             nb.erase(std::unique(nb.begin(), nb.end()), nb.end());
             for (size_t i = 0; i < nb.size(); ++i)
-                for (size_t j = i + 1; j < nb.size() && nb[j] - nb[i] < 32; ++j)
-                    out.share[nb[i]] |= 1u << (nb[j] - nb[i]);
+                for (size_t j = i + 1; j < nb.size() && nb[j] - nb[i] < 32; ++j) {
+                    const int32_t a = nb[i], b = nb[j];
+                    out.share[a] |= 1u << (b - a);
+                    // In a's and b's window, a's entry naming a later u is
+                    // left out (and b's with it when u is after b too).
+                    if (a >> 5 == b >> 5 && !(u >> 5 == a >> 5 && u > a))
+                        out.wshare[a] |= 1u << (b - a);
+                }
         }
     }
     std::vector<int32_t> mark((size_t)n, -1);

@@ -25,6 +25,7 @@ struct PackedAdjacency {
     std::vector<uint32_t> back;   // 2n
     std::vector<double> bw;
     std::vector<int32_t> bw_src;
+    std::vector<uint32_t> wshare;  // n (ProblemDev::wshare)
     bool resolve = false;         // in-window resolution enabled (ProblemDev::resolve)
     // State in registers (ProblemDev::dense) and its coupling matrix, rows of
     // dense_ld(n).

@@ -159,7 +159,7 @@ struct LaunchShape {
 
 // Arena byte offsets of one packed problem.
 struct ArenaOffsets {
-    size_t vinfo, dist, share, col, w, h, cu, cv, cw, betas, thr, back, bw, dw;
+    size_t vinfo, dist, share, wshare, col, w, h, cu, cv, cw, betas, thr, back, bw, dw;
 };
 
 }  // namespace host

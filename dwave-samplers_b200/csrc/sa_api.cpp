@@ -663,6 +663,7 @@ int b200sa_plan_create(const b200sa_problem *problems, int32_t num_problems,
         o.vinfo = take(8 * n);
         o.dist = take(n);
         o.share = take(4 * n);
+        o.wshare = take(4 * n);
         o.col = take(4 * 2 * m);
         o.w = take(8 * 2 * m);
         o.h = take(8 * n);
@@ -700,6 +701,7 @@ int b200sa_plan_create(const b200sa_problem *problems, int32_t num_problems,
             std::memcpy(&staging[o.vinfo], adj[i].vinfo.data(), 8 * n);
             std::memcpy(&staging[o.dist], adj[i].dist.data(), n);
             std::memcpy(&staging[o.share], adj[i].share.data(), 4 * n);
+            std::memcpy(&staging[o.wshare], adj[i].wshare.data(), 4 * n);
             std::memcpy(&staging[o.h], q.h, 8 * n);
             std::memcpy(&staging[o.back], adj[i].back.data(), 8 * n);
         }
@@ -738,6 +740,7 @@ int b200sa_plan_create(const b200sa_problem *problems, int32_t num_problems,
         d.vinfo = reinterpret_cast<const uint2 *>(base + o.vinfo);
         d.dist = base + o.dist;
         d.share = reinterpret_cast<const uint32_t *>(base + o.share);
+        d.wshare = reinterpret_cast<const uint32_t *>(base + o.wshare);
         d.col = reinterpret_cast<const int32_t *>(base + o.col);
         d.w = reinterpret_cast<const double *>(base + o.w);
         d.h = reinterpret_cast<const double *>(base + o.h);

@@ -190,6 +190,7 @@ struct Prob {
     const double *__restrict__ w;
     const uint8_t *__restrict__ dist;
     const uint32_t *__restrict__ share;
+    const uint32_t *__restrict__ wshare;
     int regular_degree;
     uint32_t regular_magic;
     const uint2 *__restrict__ back;
@@ -205,6 +206,7 @@ __device__ __forceinline__ Prob load_prob(const ProblemDev *P) {
     q.w = P->w;
     q.dist = P->dist;
     q.share = P->share;
+    q.wshare = P->wshare;
     q.regular_degree = P->regular_degree;
     q.regular_magic = P->regular_magic;
     q.back = P->back;
@@ -288,6 +290,11 @@ struct DeFor<kStageBand> {
 __device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" : : "r"(s), "l"(gmem) : "memory");
+}
+// The same for 16 bytes, both addresses 16-byte aligned.
+__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" : : "r"(s), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() {
     asm volatile("cp.async.commit_group;" : : : "memory");
@@ -439,12 +446,15 @@ __device__ __forceinline__ void add_group(const DE &de, int x, unsigned grp, con
 // non-adjacent.  Entries are applied lane-parallel in rounds of 32; equal
 // targets within a round are summed in entry order by their first lane.
 // `scratch` holds 32 doubles followed by 32 ints.
-template <class DE, class VAL>
+// WINDOWED: the lanes are the variables of one window, and entries naming a
+// later variable of it are left out.
+template <bool WINDOWED = false, class DE, class VAL>
 __device__ __forceinline__ void push_entries(const Prob &P, DE de, VAL val,
                                              double *scratch, unsigned fm, int v,
                                              int start, int deg, double mult,
                                              bool may_conflict, unsigned lane) {
     const bool f = (fm >> lane) & 1u;
+    [[maybe_unused]] const int w0 = v - (int)lane;
     int *owner_of_rank = reinterpret_cast<int *>(scratch + 32);
     const int D = P.regular_degree;
     int excl = 0, total;
@@ -481,24 +491,25 @@ __device__ __forceinline__ void push_entries(const Prob &P, DE de, VAL val,
                 }
                 const int e = __shfl_sync(kFull, start, k) + (t - __shfl_sync(kFull, excl, k));
                 const double m_k = __shfl_sync(kFull, mult, k);
-                nb[i] = 0;
+                nb[i] = -1;
                 x[i] = 0.0;
                 if (t < total) {
                     nb[i] = __ldg(&P.col[e]);
                     x[i] = __dmul_rn(__dmul_rn(m_k, __ldg(&P.w[e])), val(nb[i]));
+                    if (WINDOWED && nb[i] > w0 + k && nb[i] < w0 + 32) nb[i] = -1;
                 }
             }
             if constexpr (DE::kAsyncAdd) {
 #pragma unroll
                 for (int i = 0; i < 3; ++i)
-                    if (base + 32 * i + (int)lane < total) de.add(nb[i], x[i]);
+                    if (nb[i] >= 0) de.add(nb[i], x[i]);
             } else {
 #pragma unroll
                 for (int i = 0; i < 3; ++i)
-                    if (base + 32 * i + (int)lane < total) dv[i] = de.get(nb[i]);
+                    if (nb[i] >= 0) dv[i] = de.get(nb[i]);
 #pragma unroll
                 for (int i = 0; i < 3; ++i)
-                    if (base + 32 * i + (int)lane < total) de.set(nb[i], __dadd_rn(dv[i], x[i]));
+                    if (nb[i] >= 0) de.set(nb[i], __dadd_rn(dv[i], x[i]));
             }
         }
         __syncwarp();
@@ -506,7 +517,7 @@ __device__ __forceinline__ void push_entries(const Prob &P, DE de, VAL val,
     }
     for (int base = 0; base < total; base += 32) {
         const int t = base + (int)lane;
-        const bool a = t < total;
+        bool a = t < total;
         int k, e;
         if (D) {
             const int r = (int)(((uint32_t)t * P.regular_magic) >> 16);  // t / D
@@ -528,6 +539,7 @@ __device__ __forceinline__ void push_entries(const Prob &P, DE de, VAL val,
         if (a) {
             nb = __ldg(&P.col[e]);
             x = __dmul_rn(__dmul_rn(m_k, __ldg(&P.w[e])), val(nb));
+            if (WINDOWED && nb > w0 + k && nb < w0 + 32) a = false, nb = -1 - (int)lane;
         }
         const unsigned grp = may_conflict ? __match_any_sync(kFull, nb) : (1u << lane);
         const bool alone = grp == (1u << lane);
@@ -573,15 +585,23 @@ struct PreEntries {
 
 // Entry t of the flips' lists for equal-length lists (list v at v * D): its
 // target, coupling and the lane k of its flip.  `rank_tab[f]` is the lane of
-// the f-th flip in variable order.
+// the f-th flip in variable order.  STAGED: P.col and P.w hold the lists of
+// this window alone, in shared memory.
+template <bool STAGED = false>
 __device__ __forceinline__ void regular_load(const Prob &P, const int *rank_tab, int p, int t,
                                              int &k, int &nb, double &wt) {
     const int D = P.regular_degree;
     const int r = (int)(((uint32_t)t * P.regular_magic) >> 16);  // t / D
     k = rank_tab[r];
-    const int e = (p + k) * D + (t - r * D);
-    nb = __ldg(&P.col[e]);
-    wt = __ldg(&P.w[e]);
+    if constexpr (STAGED) {
+        const int e = k * D + (t - r * D);
+        nb = P.col[e];
+        wt = P.w[e];
+    } else {
+        const int e = (p + k) * D + (t - r * D);
+        nb = __ldg(&P.col[e]);
+        wt = __ldg(&P.w[e]);
+    }
 }
 
 // Neighbour updates of the committed flips for equal-length lists.  `mult` is
@@ -594,8 +614,9 @@ __device__ __forceinline__ void regular_load(const Prob &P, const int *rank_tab,
 // chunks of 32 kPreGroups whose delta-energy loads are all issued before
 // their stores, so a chunk waits on memory once.  Otherwise they go in rounds
 // of 32, equal targets within a round summed in entry order by their first
-// lane, as in apply_flips.
-template <class DE>
+// lane, as in apply_flips.  WINDOWED: entries naming a later variable of the
+// window are left out.
+template <bool WINDOWED = false, bool STAGED = false, class DE>
 __device__ __forceinline__ void update_regular(const Prob &P, DE de, const int8_t *sp,
                                                double *scratch, const int *rank_tab,
                                                int nflips, int p, bool pre, const PreEntries &pe,
@@ -613,23 +634,23 @@ __device__ __forceinline__ void update_regular(const Prob &P, DE de, const int8_
                 if (pre && base == 0) {
                     k = pe.k[i], q = pe.nb[i], wt = pe.w[i];
                 } else if (t < total) {
-                    regular_load(P, rank_tab, p, t, k, q, wt);
+                    regular_load<STAGED>(P, rank_tab, p, t, k, q, wt);
                 }
                 const double m_k = __shfl_sync(kFull, mult, k);
-                nb[i] = q;
                 x[i] = __dmul_rn(__dmul_rn(m_k, wt), (double)(int)sp[q]);
+                nb[i] = t >= total || (WINDOWED && q > p + k && q < p + 32) ? -1 : q;
             }
             if constexpr (DE::kAsyncAdd) {
 #pragma unroll
                 for (int i = 0; i < kPreGroups; ++i)
-                    if (base + 32 * i + (int)lane < total) de.add(nb[i], x[i]);
+                    if (nb[i] >= 0) de.add(nb[i], x[i]);
             } else {
 #pragma unroll
                 for (int i = 0; i < kPreGroups; ++i)
-                    if (base + 32 * i + (int)lane < total) dv[i] = de.get(nb[i]);
+                    if (nb[i] >= 0) dv[i] = de.get(nb[i]);
 #pragma unroll
                 for (int i = 0; i < kPreGroups; ++i)
-                    if (base + 32 * i + (int)lane < total) de.set(nb[i], __dadd_rn(dv[i], x[i]));
+                    if (nb[i] >= 0) de.set(nb[i], __dadd_rn(dv[i], x[i]));
             }
         }
         __syncwarp();
@@ -637,7 +658,7 @@ __device__ __forceinline__ void update_regular(const Prob &P, DE de, const int8_
     }
     for (int base = 0; base < total; base += 32) {
         const int t = base + (int)lane;
-        const bool a = t < total;
+        bool a = t < total;
         int k = 0, nb = 0;
         double wt = 0.0;
         if (pre && base == 0) {
@@ -645,15 +666,15 @@ __device__ __forceinline__ void update_regular(const Prob &P, DE de, const int8_
         } else if (pre && base == 32) {
             k = pe.k[1], nb = pe.nb[1], wt = pe.w[1];
         } else if (a) {
-            regular_load(P, rank_tab, p, t, k, nb, wt);
+            regular_load<STAGED>(P, rank_tab, p, t, k, nb, wt);
         }
         const double m_k = __shfl_sync(kFull, mult, k);
         double x = 0.0;
         if (a) {
             x = __dmul_rn(__dmul_rn(m_k, wt), (double)(int)sp[nb]);
-        } else {
-            nb = -1 - (int)lane;  // distinct per inactive lane
+            if (WINDOWED && nb > p + k && nb < p + 32) a = false;
         }
+        if (!a) nb = -1 - (int)lane;  // distinct per inactive lane
         const unsigned grp = __match_any_sync(kFull, nb);
         const bool alone = grp == (1u << lane);
         if (a && alone) de.add(nb, x);
@@ -953,16 +974,14 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
 // round per dependent flip: L = 32 lattice, 256 reads x 64 sweeps 226 -> 171 ms;
 // L = 8, 4096 x 50 5.0 -> 3.4; L = 16, 1000 x 20 11.9 -> 7.4.)
 //
-// The update phase then applies every flip's entries to the delta energies in
-// memory in entry order with the spins as they were at the start of the pass,
-// and negates the flipped variables' own delta energies last: negation is
-// exact and commutes with rounding, so a contribution added after the negation
-// in the reference (a neighbour that flipped earlier) equals the negated
-// contribution added before it.
+// The update phase writes the window's own delta energies and spins first: they
+// hold the contributions of the earlier flips and the variable's own negation.
+// Then it applies every flip's other entries in variable order: those naming
+// an earlier variable of the window or one outside it.
 //
 // Delta energies on chip or in the band: the next window's records are loaded
 // into registers while this one is worked on (a window always starts 32
-// further on), its lists brought into L1.
+// further on).
 template <bool GIBBS, int STAGE>
 __device__ __forceinline__ void sweep_resolved(const Prob &P, double *de_g, int8_t *sp,
                                                double *scratch, uint64_t *ring, RingState &rs,
@@ -991,7 +1010,7 @@ __device__ __forceinline__ void sweep_resolved(const Prob &P, double *de_g, int8
     auto load = [&](int v) {
         Record r{0u, make_uint2(0u, 0u), make_uint2(0u, 0u), 0.0};
         if (v < n) {
-            r.shr = __ldg(&P.share[v]);
+            r.shr = __ldg(&P.wshare[v]);
             r.vi = D ? make_uint2((uint32_t)v * (uint32_t)D, (uint32_t)D) : __ldg(&P.vinfo[v]);
             r.bk = __ldg(&P.back[v]);
         }
@@ -1002,6 +1021,32 @@ __device__ __forceinline__ void sweep_resolved(const Prob &P, double *de_g, int8
     };
     Record next = load((int)lane);
     load_near(next);
+    // Equal lists and a band: the next window's lists (whole 16-byte pieces)
+    // are copied into one of two buffers behind the band while this window is
+    // worked on; they land with the band's next slide.  (Loads of them in the
+    // update phase waited on L2, a quarter of the pass: prefetch.global.L1 does
+    // not bring a line into L1 here.  With the left-out entries, which remove
+    // most conflicts, L = 32, 256 reads x 64 sweeps 171 -> 147 ms, L = 16, 1000 x
+    // 20 7.4 -> 6.4.)
+    [[maybe_unused]] const bool staged = BANDED && band_w > 0 && D > 0 && D <= kListMaxDegree;
+    [[maybe_unused]] double *list_w = band + band_w;
+    [[maybe_unused]] int32_t *list_col =
+        reinterpret_cast<int32_t *>(list_w + 2 * 32 * kListMaxDegree);
+    [[maybe_unused]] auto stage = [&](int p) {
+        const int entries = min(32, n - p) * D;
+        const double *w = P.w + (int64_t)p * D;
+        const int32_t *col = P.col + (int64_t)p * D;
+        double *to_w = list_w + (p & 32) * D;
+        int32_t *to_col = list_col + (p & 32) * D;
+        for (int i = (int)lane; 2 * i < entries; i += 32) cp_async16(to_w + 2 * i, w + 2 * i);
+        for (int i = (int)lane; 4 * i < entries; i += 32) cp_async16(to_col + 4 * i, col + 4 * i);
+    };
+    if constexpr (BANDED) {
+        if (staged) {
+            stage(0);
+            cp_async_commit();
+        }
+    }
     for (int b = 0; b < reload(P.pd->num_betas); ++b) {
         const double beta = __ldg(&reload(P.pd->betas)[b]);
         const double thr = __ldg(&reload(P.pd->thresholds)[b]);
@@ -1033,16 +1078,15 @@ __device__ __forceinline__ void sweep_resolved(const Prob &P, double *de_g, int8
                     r = next;
                     const int vn = p + 32 < n ? v + 32 : (int)lane;
                     next = load(vn);
-                    const uint32_t e0 = D ? next.vi.x : r.vi.x;
-                    if ((D ? vn : v) < n) {
-                        prefetch_l1(P.col + e0);
-                        prefetch_l1(P.w + e0);
+                    if constexpr (BANDED) {
+                        if (staged && p + 32 < n) stage(p + 32);
                     }
                 } else {
                     r = load(v);
                     load_near(r);
                 }
                 double d = d0;
+                unsigned rel = 0u;  // flipped lanes before this one, as d holds them
                 Choice<GIBBS> ch;
                 ch.look(d, scale, thr, act);
                 unsigned fm = 0u, ties = 0u;
@@ -1053,7 +1097,6 @@ __device__ __forceinline__ void sweep_resolved(const Prob &P, double *de_g, int8
                     const unsigned back = act ? __brev(r.bk.x) >> (31u - lane) : 0u;
                     const int o_near = r.bk.x ? __ffs(r.bk.x) - 1 : 0;
                     const unsigned up = __ballot_sync(kFull, s_cur > 0);
-                    unsigned rel = 0u;  // flipped lanes among `back`, as d holds them
                     unsigned nm;
                     for (;;) {
                         nm = __ballot_sync(kFull, ch.need);
@@ -1101,28 +1144,43 @@ __device__ __forceinline__ void sweep_resolved(const Prob &P, double *de_g, int8
                             __syncwarp();
                         }
                     }
-                    // A slot can receive two additions only through a
-                    // neighbour common to two flips.
+                    // A slot can receive two of the additions below only
+                    // through a neighbour common to two flips.
                     const unsigned later = lane < 31 ? fm >> (lane + 1) : 0u;
                     const bool f = (fm >> lane) & 1u;
                     const bool may_conflict = __any_sync(kFull, f && ((r.shr >> 1) & later));
+                    // cpu_sa.cpp:189-190, the contributions of the window's
+                    // earlier flips included.
+                    if (f || rel) de.set(v, f ? -d : d);
+                    if (f) sp[v] = (int8_t)(-s_cur);
+                    const double mult = (double)(4 * s_cur);
                     if (D) {
                         if (f) rank_tab[__popc(fm & lt_mask)] = (int)lane;
                         __syncwarp();
                         const PreEntries none{};
-                        update_regular(P, de, sp, scratch, rank_tab, __popc(fm), p, false, none,
-                                       may_conflict, (double)(4 * s_cur), lane);
-                        if (f) {  // cpu_sa.cpp:189-190, after the variable's own updates
-                            sp[v] = (int8_t)(-s_cur);
-                            de.set(v, -de.get(v));
+                        if (BANDED && staged) {
+                            Prob W = P;
+                            W.col = list_col + (p & 32) * D;
+                            W.w = list_w + (p & 32) * D;
+                            update_regular<true, BANDED>(W, de, sp, scratch, rank_tab, __popc(fm),
+                                                         p, false, none, may_conflict, mult, lane);
+                        } else {
+                            update_regular<true>(P, de, sp, scratch, rank_tab, __popc(fm), p,
+                                                 false, none, may_conflict, mult, lane);
                         }
-                        __syncwarp();
                     } else {
-                        apply_flips(P, de, sp, scratch, fm, v, (int)r.vi.x,
-                                    (int)(r.vi.y & kDegMask), s_cur, may_conflict, lane);
+                        __syncwarp();
+                        push_entries<true>(P, de, [&](int x) { return (double)(int)sp[x]; },
+                                           scratch, fm, v, (int)r.vi.x, (int)(r.vi.y & kDegMask),
+                                           mult, may_conflict, lane);
                     }
                 }
                 if constexpr (BANDED) {
+                    // (Window 0's buffer may be this last window's.)
+                    if (staged && p + 32 >= n) {
+                        __syncwarp();
+                        stage(0);
+                    }
                     const int c = min(32, n - p);
                     if (band_w) band_slide(de, n, p, band_b, c, lane);
                     de.lo = p + c - band_b;

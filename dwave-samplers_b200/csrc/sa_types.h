@@ -76,6 +76,9 @@ struct ProblemDev {
     int32_t dense;
     const uint2 *back;
     const double *bw;
+    // The conflict mask (share) of windows of 32 variables from a multiple of 32
+    // on, without entries naming a later variable of the same window.
+    const uint32_t *wshare;
     const double *dense_w;
     // Banded delta energies (kStageBand): adjacency entries mostly within
     // band_b of their variable; band_w is the shared-memory ring size (a power
@@ -87,6 +90,10 @@ constexpr int kDenseSlots = 10;  // variables per lane at most
 constexpr int kDenseMaxN = 32 * kDenseSlots;
 __host__ __device__ inline int dense_ld(int n) { return (n + 31) & ~31; }
 constexpr int kBandMaxSlots = 8192;  // 64 KB of delta energies per warp at most
+// Equal lists up to this length are staged beside the band, two windows of
+// them (12 bytes an entry).
+constexpr int kListMaxDegree = 8;
+constexpr int kListBytes = 2 * 32 * kListMaxDegree * 12;
 
 // Per-read counters written by the kernel.
 struct ReadStats {
@@ -278,7 +285,7 @@ constexpr int kNumStages = 4;
 inline int region_bytes_for_stage(int stage, int cap_n, int band_cap = 0) {
     if (stage == kStageShared) return region_bytes_for(cap_n);
     if (stage == kStageSpins) return kRing * 8 + kScratchBytes + ((cap_n + 15) & ~15);
-    if (stage == kStageBand) return kRing * 8 + kScratchBytes + ((cap_n + 15) & ~15) + 8 * band_cap;
+    if (stage == kStageBand) return kRing * 8 + kScratchBytes + ((cap_n + 15) & ~15) + 8 * band_cap + kListBytes;
     return kRing * 8 + kScratchBytes;
 }
 

@@ -29,7 +29,8 @@ def graph(kind, size):
 
 @pytest.mark.parametrize("rule", ["Metropolis", "Gibbs"])
 @pytest.mark.parametrize("kind,size,R", [("chain", 129, 9), ("chain", 2001, 300), ("lattice", 6, 20),
-                                         ("lattice", 11, 9), ("lattice", 21, 3), ("lattice", 32, 2),
+                                         ("lattice", 11, 9), ("lattice", 21, 3), ("lattice", 22, 3),
+                                         ("lattice", 32, 2),
                                          ("dense", 330, 5), ("near", 400, 20), ("near", 9000, 3)])
 def test_resolved_windows(kind, size, R, rule):
     n, u, v, J = graph(kind, size)
