@@ -815,6 +815,7 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
     const int n = P.n;
     const int D = P.regular_degree;
     const unsigned lt_mask = (1u << lane) - 1u;
+    const float inf = __int_as_float(0x7f800000);
     int *rank_tab = reinterpret_cast<int *>(scratch + 32);
     typename DeFor<STAGE>::T de;
     bool band_live = false;
@@ -825,6 +826,7 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
     for (int b = 0; b < reload(P.pd->num_betas); ++b) {
         const double beta = __ldg(&reload(P.pd->betas)[b]);
         const double thr = __ldg(&reload(P.pd->thresholds)[b]);
+        const float scale = Choice<GIBBS>::scale(beta);
         for (int sw = 0; sw < reload(P.pd->sweeps_per_beta); ++sw) {
             SweepCount cnt;
             if constexpr (BANDED) {
@@ -868,18 +870,28 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
                         if (!D) prefetch_l1(P.vinfo + vn);
                     }
                 }
-                const bool consider = act && !(d >= thr);  // cpu_sa.cpp:140
-                const bool need = GIBBS ? consider : (consider && !(d <= 0.0));
-                const unsigned nm = __ballot_sync(kFull, need);
-                bool acc = GIBBS ? false : consider;  // Metropolis: d <= 0 accepts
-                bool near = false;
-                if (need) {
-                    const uint64_t r = ring[(rs.q + (uint32_t)__popc(nm & lt_mask)) & (kRing - 1)];
-                    const int x = decide<GIBBS>(d, beta, r);
-                    acc = (x & 1) != 0;
-                    near = (x & 2) != 0;
+                // cpu_sa.cpp:140-166.  (All lanes take a draw's logarithm and
+                // compare; a branch for those that need one measured 2-3%
+                // slower on the uneven batch.)
+                Choice<GIBBS> ch;
+                ch.look(d, scale, thr, act);
+                const unsigned nm = __ballot_sync(kFull, ch.need);
+                unsigned am = 0u, ties = 0u;
+                // (A bound of NaN counts as a decision to be made.)
+                if (__any_sync(kFull, !(ch.t == -inf))) {
+                    const int at = __popc(nm & lt_mask);
+                    const float y = draw_log2(ring[(rs.q + lane) & (kRing - 1)]);
+                    const float gap = ch.t - __shfl_sync(kFull, y, at);
+                    am = __ballot_sync(kFull, gap > kBand);
+                    if (__any_sync(kFull, !(fabsf(gap) > kBand))) {  // inside the band
+                        int x = 0;
+                        if (!(fabsf(gap) > kBand))
+                            x = ch.exact(d, beta, ring[(rs.q + (uint32_t)at) & (kRing - 1)]);
+                        am |= __ballot_sync(kFull, (x & 1) != 0);
+                        ties = __ballot_sync(kFull, (x & 2) != 0);
+                    }
                 }
-                const unsigned am = __ballot_sync(kFull, acc);
+                const bool acc = (am >> lane) & 1u;
                 // Equal-length lists: start loading the accepted flips'
                 // adjacency before the commit point is known.
                 const double mult = (double)(int)(int8_t)(4 * s_cur);
@@ -897,13 +909,11 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
                     }
                 }
                 const int bound = acc ? (int)lane + dist : 32;
-                const int c = min(__reduce_min_sync(kFull, bound), L);
+                const int c = am ? min(__reduce_min_sync(kFull, bound), L) : L;
                 const unsigned done = c >= 32 ? kFull : ((1u << c) - 1u);
-                const uint32_t used = (uint32_t)__popc(nm & done);
                 const unsigned fm = am & done;
-                const unsigned nearm = __ballot_sync(kFull, near) & done;
-                rs.q += used;
-                cnt.pass((unsigned)__popc(fm), (unsigned)__popc(nearm));
+                rs.q += (uint32_t)__popc(nm & done);
+                cnt.pass((unsigned)__popc(fm), (unsigned)__popc(ties & done));
                 if constexpr (BANDED) {
                     // The slots the last slide fetched lie at the far end of
                     // the band, which only an update through a coupler longer
