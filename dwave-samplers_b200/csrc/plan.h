@@ -182,6 +182,7 @@ struct b200sa_plan_s {
     std::vector<int32_t> n, reads, sweeps;  // per problem
     std::vector<int64_t> state_off, read_off;
     int64_t total_state = 0, total_reads = 0;
+    bool any_dup = false;  // some problem's list names a target twice
     int32_t max_n = 0;
     b200sa::host::DevArray<uint8_t> arena;
     b200sa::host::DevArray<b200sa::ProblemDev> dprobs;

@@ -681,6 +681,7 @@ int b200sa_plan_create(const b200sa_problem *problems, int32_t num_problems,
         P->reads.push_back(q.num_reads);
         P->sweeps.push_back(q.sweeps_per_beta * q.num_betas);
         P->max_n = std::max(P->max_n, q.num_vars);
+        P->any_dup = P->any_dup || adj[i].any_dup;
     }
     P->total_state = P->state_off[num_problems];
     P->total_reads = P->read_off[num_problems];

@@ -292,7 +292,7 @@ static SdKernel sd_kernel_for(bool sparse, bool smem) {
 cudaError_t launch_sd(bool sparse, bool smem, const SdArgs &args, int grid, int warps_per_cta,
                       int region_bytes, cudaStream_t stream) {
     const SdKernel k = sd_kernel_for(sparse, smem);
-    const size_t bytes = (size_t)warps_per_cta * (size_t)region_bytes;
+    const size_t bytes = (size_t)args.table_bytes + (size_t)warps_per_cta * (size_t)region_bytes;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return e;
     k<<<grid, warps_per_cta * 32, bytes, stream>>>(args, warps_per_cta, region_bytes);
@@ -300,9 +300,9 @@ cudaError_t launch_sd(bool sparse, bool smem, const SdArgs &args, int grid, int 
 }
 
 cudaError_t sd_occupancy(bool sparse, bool smem, int warps_per_cta, int region_bytes,
-                         int *ctas_per_sm) {
+                         int table_bytes, int *ctas_per_sm) {
     const SdKernel k = sd_kernel_for(sparse, smem);
-    const size_t bytes = (size_t)warps_per_cta * (size_t)region_bytes;
+    const size_t bytes = (size_t)table_bytes + (size_t)warps_per_cta * (size_t)region_bytes;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, k, warps_per_cta * 32, bytes);

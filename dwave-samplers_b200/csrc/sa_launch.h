@@ -57,7 +57,7 @@ cudaError_t kernel_occupancy(int variant, int warps_per_cta, int region_bytes,
 cudaError_t launch_sd(bool sparse, bool smem, const SdArgs &args, int grid, int warps_per_cta,
                       int region_bytes, cudaStream_t stream);
 cudaError_t sd_occupancy(bool sparse, bool smem, int warps_per_cta, int region_bytes,
-                         int *ctas_per_sm);
+                         int table_bytes, int *ctas_per_sm);
 // Rotor kernel; `stage` is its state location (kStageShared only for the
 // proposals that keep delta energies, 0 and 1).
 cudaError_t launch_rmc(bool random_order, int proposal, int stage, const RmcArgs &args, int grid,

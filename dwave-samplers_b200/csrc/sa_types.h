@@ -145,14 +145,24 @@ struct SdArgs {
     double *scratch_fe;          // else per-warp global slots
     int8_t *scratch_s;
     int64_t scratch_stride;
+    int32_t table_bytes;         // list starts at the head of a CTA's shared memory
+    int32_t any_dup;             // some list names a target twice
+    unsigned long long *scratch_key;  // group minima (sd_kernel.cuh)
+    uint8_t *scratch_at;
+    int64_t group_stride;
     unsigned long long *capped;  // samples stopped by max_steps
 };
 
 // Per-warp shared region of the descent kernel: 32 doubles for equal-target
-// sums, then (state in shared memory) flip energies and spins.
+// sums, then (state in shared memory) flip energies, group keys, spins and the
+// places of the group minima.
 constexpr int kSdScratchBytes = 32 * 8;  // equal-target sums
-inline int sd_region_bytes(int cap_n) {
-    return kSdScratchBytes + cap_n * 8 + ((cap_n + 15) & ~15);
+// List starts, one table per CTA (state in shared memory, lists of different
+// lengths).
+inline int64_t sd_table_bytes(int64_t n) { return (4 * (n + 1) + 15) & ~int64_t(15); }
+inline int64_t sd_region_bytes(int64_t cap_n) {
+    const int64_t groups = (cap_n + 31) / 32;
+    return (kSdScratchBytes + 8 * (cap_n + groups) + cap_n + groups + 15) & ~int64_t(15);
 }
 
 // Arguments of the rotor-model annealing kernel (rmc_kernel.cuh).
