@@ -129,10 +129,13 @@ inline int size_class(int n, int onchip_max) {
 }
 
 // Kernel kind of a problem: bit 0 Gibbs, bit 1 random order, bit 2
-// in-window resolution (sequential order only), bit 3 state in registers.
+// in-window resolution (sequential order only), bit 3 state in registers, bit 4
+// equal list lengths.
 inline int kind_of(const ProblemDev &d) {
     return (d.proposal == 0 ? kKindGibbs : 0) | (d.varorder ? kKindRandom : 0) |
-           (d.dense ? kKindDense : d.resolve && !d.varorder ? kKindResolve : 0);
+           (d.dense ? kKindDense
+                    : (d.resolve && !d.varorder ? kKindResolve : 0) |
+                          (d.regular_degree ? kKindRegular : 0));
 }
 
 // Launch configuration of one bucket chosen by the autotuner (unset: the

@@ -75,7 +75,7 @@ std::string tune_key(const b200sa_plan_s *P, int kind, int max_n, int mean_degre
     const int n_bin = (max_n + 63) / 64 * 64;
     std::ostringstream k;
     k << "gpu=" << name << ";sms=" << P->prop.multiProcessorCount << ";lib=" << b200sa_version()
-      << ";kind=" << kind << ";n=" << n_bin << ";deg=" << mean_degree;
+      << ";kind=" << (kind & ~kKindRegular) << ";n=" << n_bin << ";deg=" << mean_degree;
     std::string s = k.str();
     for (char &c : s)
         if (c == ' ') c = '_';

@@ -95,12 +95,12 @@ __device__ __forceinline__ double rmc_field(const RmcWarp<DE> &W, int var) {
 
 // The committed reflections `fm` of a window: neighbour updates (:270-283),
 // then each flip's own delta energy -d and angle.
-template <class DE>
+template <bool REG, class DE>
 __device__ __forceinline__ void rmc_reflect(RmcWarp<DE> &W, unsigned fm, int v, uint2 vi,
                                             uint8_t cur, double d, bool may_conflict) {
     const uint8_t prop = (uint8_t)(128 + cur);
     const double mult = __dmul_rn(2.0, __dsub_rn(W.cs[cur], W.cs[prop]));
-    push_entries(W.P, W.de, [&](int x) { return W.cs[W.st[x]]; }, W.scratch, fm, v, (int)vi.x,
+    push_entries<REG>(W.P, W.de, [&](int x) { return W.cs[W.st[x]]; }, W.scratch, fm, v, (int)vi.x,
                  (int)vi.y, mult, may_conflict, W.lane);
     if ((fm >> W.lane) & 1u) {
         W.st[v] = prop;
@@ -155,7 +155,10 @@ __device__ __forceinline__ void rmc_reflect_sequential(RmcWarp<DE> &W, RingState
             const bool f = (fm >> lane) & 1u;
             const bool may_conflict =
                 __any_sync(kFull, f && ((shr & 1u) || ((shr >> 1) & later)));
-            rmc_reflect(W, fm, v, vi, cur, d, may_conflict);
+            if (P.regular_degree)
+                rmc_reflect<true>(W, fm, v, vi, cur, d, may_conflict);
+            else
+                rmc_reflect<false>(W, fm, v, vi, cur, d, may_conflict);
         }
         p += c;
     }
@@ -206,7 +209,10 @@ __device__ __forceinline__ void rmc_reflect_random(RmcWarp<DE> &W, RingState &rs
             const uint2 vi = __ldg(&P.vinfo[var]);
             const uint8_t cur = W.st[var];
             __syncwarp();
-            rmc_reflect(W, fm, var, vi, cur, d, true);
+            if (P.regular_degree)
+                rmc_reflect<true>(W, fm, var, vi, cur, d, true);
+            else
+                rmc_reflect<false>(W, fm, var, vi, cur, d, true);
         }
     }
 }

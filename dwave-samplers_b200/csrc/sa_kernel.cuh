@@ -439,6 +439,56 @@ __device__ __forceinline__ void add_group(const DE &de, int x, unsigned grp, con
     }
 }
 
+// The flips of `rest` without an earlier flip in it that shares a neighbour
+// (`shr` is the lane's conflict mask, ProblemDev::share): applied together they
+// name no slot twice, and applied before the others they keep the order of
+// additions.
+__device__ __forceinline__ unsigned first_phase(unsigned rest, uint32_t shr, unsigned lane) {
+    unsigned partners = 0u;
+    if (lane < 31 && ((rest >> lane) & 1u))
+        partners = ((shr >> 1) & (rest >> (lane + 1))) << (lane + 1);
+    return rest & ~__reduce_or_sync(kFull, partners);
+}
+
+// Adds x[i] to slot nb[i] (none when negative) of N entries per lane, entry i
+// belonging to the flip of lane k[i], in phases (first_phase) with a barrier
+// between two of them, so additions to one slot from different lanes land in
+// the order of the phases.  What is left after kPhases of them (hubs that most
+// flips share) is matched, 32 entries at a time.
+constexpr int kPhases = 3;
+template <int N, class DE>
+__device__ __forceinline__ void add_phased(const DE &de, const int (&nb)[N], const double (&x)[N],
+                                           const int (&k)[N], unsigned fm, uint32_t shr,
+                                           double *scratch, unsigned lane) {
+    unsigned rest = fm;
+    for (int phase = 0; phase < kPhases && rest; ++phase) {
+        const unsigned now = first_phase(rest, shr, lane);
+        bool on[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) on[i] = nb[i] >= 0 && ((now >> k[i]) & 1u);
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if (on[i]) de.add(nb[i], x[i]);
+        __syncwarp();
+        rest &= ~now;
+    }
+    if (!rest) return;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const bool on = nb[i] >= 0 && ((rest >> k[i]) & 1u);
+        const unsigned grp = __match_any_sync(kFull, on ? nb[i] : -1 - (int)lane);
+        const bool alone = grp == (1u << lane);
+        if (on && alone) de.add(nb[i], x[i]);
+        if (__any_sync(kFull, on && !alone)) {
+            scratch[lane] = x[i];
+            __syncwarp();
+            if (on && !alone && lane == (unsigned)(__ffs(grp) - 1))
+                add_group(de, nb[i], grp, scratch);
+        }
+        __syncwarp();
+    }
+}
+
 // The neighbour updates of every lane whose bit is set in `fm`: slot x gets
 // (mult * J) * val(x) for each entry (x, J) of the lane's list.  Lane k of the
 // warp holds its variable v, list start `start`, degree `deg` and factor
@@ -448,17 +498,23 @@ __device__ __forceinline__ void add_group(const DE &de, int x, unsigned grp, con
 // `scratch` holds 32 doubles followed by 32 ints.
 // WINDOWED: the lanes are the variables of one window, and entries naming a
 // later variable of it are left out.
-template <bool WINDOWED = false, class DE, class VAL>
+// REG: lists of one length.
+// PHASED: in global slots, lists of different lengths whose flips may share
+// neighbours go in phases (add_phased) instead of being matched 32 entries at
+// a time: 500 reads x 20 Gibbs sweeps of a sparse n = 4000, degree 12 problem
+// 7.0 -> 6.2 ms.  (Slower so: equal lists, 2% on the uneven batch, and state in
+// shared memory, n = 400, 5%.)
+template <bool REG, bool WINDOWED = false, bool PHASED = false, class DE, class VAL>
 __device__ __forceinline__ void push_entries(const Prob &P, DE de, VAL val,
                                              double *scratch, unsigned fm, int v,
                                              int start, int deg, double mult,
-                                             bool may_conflict, unsigned lane) {
+                                             bool may_conflict, unsigned lane, uint32_t shr = 0u) {
     const bool f = (fm >> lane) & 1u;
     [[maybe_unused]] const int w0 = v - (int)lane;
     int *owner_of_rank = reinterpret_cast<int *>(scratch + 32);
-    const int D = P.regular_degree;
+    const int D = REG ? P.regular_degree : 0;
     int excl = 0, total;
-    if (D) {
+    if constexpr (REG) {
         // Equal list lengths: entry t belongs to the (t / D)-th flip.
         if (f) owner_of_rank[__popc(fm & ((1u << lane) - 1u))] = (int)lane;
         total = __popc(fm) * D;
@@ -474,11 +530,14 @@ __device__ __forceinline__ void push_entries(const Prob &P, DE de, VAL val,
         excl = incl - my;
         total = __shfl_sync(kFull, incl, 31);
     }
-    if (!may_conflict && !D) {
+    // (shr bit 0: a list names a target twice.)
+    const bool phased = PHASED && DE::kAsyncAdd && may_conflict && !REG &&
+                        !__any_sync(kFull, f && (shr & 1u));
+    if (!REG && (!may_conflict || phased)) {
         // No two entries name the same slot: each chunk of 96 entries issues
         // all of its delta-energy loads before its stores.
         for (int base = 0; base < total; base += 96) {
-            int nb[3];
+            int nb[3], kk[3];
             double x[3], dv[3];
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
@@ -491,6 +550,7 @@ __device__ __forceinline__ void push_entries(const Prob &P, DE de, VAL val,
                 }
                 const int e = __shfl_sync(kFull, start, k) + (t - __shfl_sync(kFull, excl, k));
                 const double m_k = __shfl_sync(kFull, mult, k);
+                kk[i] = k;
                 nb[i] = -1;
                 x[i] = 0.0;
                 if (t < total) {
@@ -499,7 +559,9 @@ __device__ __forceinline__ void push_entries(const Prob &P, DE de, VAL val,
                     if (WINDOWED && nb[i] > w0 + k && nb[i] < w0 + 32) nb[i] = -1;
                 }
             }
-            if constexpr (DE::kAsyncAdd) {
+            if (PHASED && DE::kAsyncAdd && phased) {
+                add_phased<3>(de, nb, x, kk, fm, shr, scratch, lane);
+            } else if constexpr (DE::kAsyncAdd) {
 #pragma unroll
                 for (int i = 0; i < 3; ++i)
                     if (nb[i] >= 0) de.add(nb[i], x[i]);
@@ -519,7 +581,7 @@ __device__ __forceinline__ void push_entries(const Prob &P, DE de, VAL val,
         const int t = base + (int)lane;
         bool a = t < total;
         int k, e;
-        if (D) {
+        if constexpr (REG) {
             const int r = (int)(((uint32_t)t * P.regular_magic) >> 16);  // t / D
             k = a ? owner_of_rank[r] : 0;
             e = __shfl_sync(kFull, v, k) * D + (t - r * D);
@@ -558,14 +620,15 @@ __device__ __forceinline__ void push_entries(const Prob &P, DE de, VAL val,
 // cpu_sa.cpp:168-191 for the flips `fm` (see push_entries); `s_old` is the
 // lane's spin.  With `own_fresh`, no entry of this pass names the lane's own
 // slot, which then still holds `d_own`.
-template <class DE>
+template <bool REG, bool PHASED = false, class DE>
 __device__ __forceinline__ void apply_flips(const Prob &P, DE de, int8_t *sp,
                                             double *scratch, unsigned fm, int v,
                                             int start, int deg, int s_old,
                                             bool may_conflict, unsigned lane,
-                                            bool own_fresh = false, double d_own = 0.0) {
-    push_entries(P, de, [&](int x) { return (double)(int)sp[x]; }, scratch, fm, v, start, deg,
-                 (double)(int)(int8_t)(4 * s_old), may_conflict, lane);
+                                            bool own_fresh = false, double d_own = 0.0,
+                                            uint32_t shr = 0u) {
+    push_entries<REG, false, PHASED>(P, de, [&](int x) { return (double)(int)sp[x]; }, scratch, fm, v, start, deg,
+                 (double)(int)(int8_t)(4 * s_old), may_conflict, lane, shr);
     if ((fm >> lane) & 1u) {  // cpu_sa.cpp:189-190, after the variable's own updates
         sp[v] = (int8_t)(-s_old);
         de.set(v, __dmul_rn(own_fresh ? d_own : de.get(v), -1.0));
@@ -805,7 +868,7 @@ __device__ __forceinline__ void band_slide(const BandDe &de, int n, int p, int b
     __syncwarp();
 }
 
-template <bool GIBBS, int STAGE>
+template <bool GIBBS, int STAGE, bool REG>
 __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
                                                  int8_t *sp, double *scratch,
                                                  uint64_t *ring, RingState &rs,
@@ -813,7 +876,7 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
                                                  int band_b) {
     constexpr bool BANDED = STAGE == kStageBand;
     const int n = P.n;
-    const int D = P.regular_degree;
+    const int D = REG ? P.regular_degree : 0;
     const unsigned lt_mask = (1u << lane) - 1u;
     const float inf = __int_as_float(0x7f800000);
     int *rank_tab = reinterpret_cast<int *>(scratch + 32);
@@ -854,7 +917,7 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
                     d = de.get(v);
                     dist = __ldg(&P.dist[v]);
                     shr = __ldg(&P.share[v]);
-                    if (!D) vi = __ldg(&P.vinfo[v]);
+                    if (!REG) vi = __ldg(&P.vinfo[v]);
                     s_cur = (int)sp[v];
                 }
                 if (act) {
@@ -867,7 +930,7 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
                     if (vn < n && !DeFor<STAGE>::T::kAsyncAdd) {
                         prefetch_l1(P.dist + vn);
                         prefetch_l1(P.share + vn);
-                        if (!D) prefetch_l1(P.vinfo + vn);
+                        if (!REG) prefetch_l1(P.vinfo + vn);
                     }
                 }
                 // cpu_sa.cpp:140-166.  (All lanes take a draw's logarithm and
@@ -898,7 +961,7 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
                 PreEntries pe;
 #pragma unroll
                 for (int i = 0; i < kPreGroups; ++i) pe.nb[i] = 0, pe.k[i] = 0, pe.w[i] = 0.0;
-                if (D && am) {
+                if (REG && am) {
                     if (acc) rank_tab[__popc(am & lt_mask)] = (int)lane;
                     __syncwarp();
                     const int pre_n = min(__popc(am) * D, 32 * kPreGroups);
@@ -936,7 +999,7 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
                     // still holds the window value d and the negation needs no
                     // load.
                     const bool own_fresh = !(shr & 1u);
-                    if (D) {
+                    if constexpr (REG) {
                         update_regular(P, de, sp, scratch, rank_tab, __popc(fm), p, true, pe,
                                        may_conflict, mult, lane);
                         if (f) {  // cpu_sa.cpp:189-190, after the variable's own updates
@@ -945,9 +1008,9 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
                         }
                         __syncwarp();
                     } else {
-                        apply_flips(P, de, sp, scratch, fm, v, (int)vi.x,
-                                    (int)(vi.y & kDegMask), s_cur, may_conflict, lane, own_fresh,
-                                    d);
+                        apply_flips<REG, true>(P, de, sp, scratch, fm, v, (int)vi.x,
+                                               (int)(vi.y & kDegMask), s_cur, may_conflict, lane,
+                                          own_fresh, d, shr);
                     }
                 }
                 if constexpr (BANDED) {
@@ -992,7 +1055,7 @@ __device__ __forceinline__ void sweep_sequential(const Prob &P, double *de_g,
 // Delta energies on chip or in the band: the next window's records are loaded
 // into registers while this one is worked on (a window always starts 32
 // further on).
-template <bool GIBBS, int STAGE>
+template <bool GIBBS, int STAGE, bool REG>
 __device__ __forceinline__ void sweep_resolved(const Prob &P, double *de_g, int8_t *sp,
                                                double *scratch, uint64_t *ring, RingState &rs,
                                                unsigned lane, double *band, int band_w,
@@ -1000,7 +1063,7 @@ __device__ __forceinline__ void sweep_resolved(const Prob &P, double *de_g, int8
     constexpr bool BANDED = STAGE == kStageBand;
     constexpr bool AHEAD = !DeFor<STAGE>::T::kAsyncAdd;
     const int n = P.n;
-    const int D = P.regular_degree;
+    const int D = REG ? P.regular_degree : 0;
     const unsigned lt_mask = (1u << lane) - 1u;
     const float inf = __int_as_float(0x7f800000);
     int *rank_tab = reinterpret_cast<int *>(scratch + 32);
@@ -1021,7 +1084,7 @@ __device__ __forceinline__ void sweep_resolved(const Prob &P, double *de_g, int8
         Record r{0u, make_uint2(0u, 0u), make_uint2(0u, 0u), 0.0};
         if (v < n) {
             r.shr = __ldg(&P.wshare[v]);
-            r.vi = D ? make_uint2((uint32_t)v * (uint32_t)D, (uint32_t)D) : __ldg(&P.vinfo[v]);
+            r.vi = REG ? make_uint2((uint32_t)v * (uint32_t)D, (uint32_t)D) : __ldg(&P.vinfo[v]);
             r.bk = __ldg(&P.back[v]);
         }
         return r;
@@ -1038,7 +1101,7 @@ __device__ __forceinline__ void sweep_resolved(const Prob &P, double *de_g, int8
     // not bring a line into L1 here.  With the left-out entries, which remove
     // most conflicts, L = 32, 256 reads x 64 sweeps 171 -> 147 ms, L = 16, 1000 x
     // 20 7.4 -> 6.4.)
-    [[maybe_unused]] const bool staged = BANDED && band_w > 0 && D > 0 && D <= kListMaxDegree;
+    [[maybe_unused]] const bool staged = BANDED && REG && band_w > 0 && D <= kListMaxDegree;
     [[maybe_unused]] double *list_w = band + band_w;
     [[maybe_unused]] int32_t *list_col =
         reinterpret_cast<int32_t *>(list_w + 2 * 32 * kListMaxDegree);
@@ -1164,7 +1227,7 @@ __device__ __forceinline__ void sweep_resolved(const Prob &P, double *de_g, int8
                     if (f || rel) de.set(v, f ? -d : d);
                     if (f) sp[v] = (int8_t)(-s_cur);
                     const double mult = (double)(4 * s_cur);
-                    if (D) {
+                    if constexpr (REG) {
                         if (f) rank_tab[__popc(fm & lt_mask)] = (int)lane;
                         __syncwarp();
                         const PreEntries none{};
@@ -1180,9 +1243,9 @@ __device__ __forceinline__ void sweep_resolved(const Prob &P, double *de_g, int8
                         }
                     } else {
                         __syncwarp();
-                        push_entries<true>(P, de, [&](int x) { return (double)(int)sp[x]; },
+                        push_entries<REG, true, true>(P, de, [&](int x) { return (double)(int)sp[x]; },
                                            scratch, fm, v, (int)r.vi.x, (int)(r.vi.y & kDegMask),
-                                           mult, may_conflict, lane);
+                                           mult, may_conflict, lane, r.shr);
                     }
                 }
                 if constexpr (BANDED) {
@@ -1308,13 +1371,13 @@ __device__ __forceinline__ int random_commit(const Prob &P, int D, uint32_t *tou
 // in a per-warp bitmap (`touch`, n bits, clear between passes).  Committed
 // flips are pairwise distinct and non-adjacent, so their neighbour updates
 // are applied together, equal targets summed in entry order.
-template <bool GIBBS, class DE>
+template <bool GIBBS, bool REG, class DE>
 __device__ __forceinline__ void sweep_random(const Prob &P, DE de,
                                              int8_t *sp, double *scratch,
                                              uint64_t *ring, RingState &rs,
                                              unsigned lane, uint32_t *touch) {
     const int n = P.n;
-    const int D = P.regular_degree;
+    const int D = REG ? P.regular_degree : 0;
     for (int b = 0; b < reload(P.pd->num_betas); ++b) {
         const double beta = __ldg(&reload(P.pd->betas)[b]);
         const double thr = __ldg(&reload(P.pd->thresholds)[b]);
@@ -1369,7 +1432,7 @@ __device__ __forceinline__ void sweep_random(const Prob &P, DE de,
                     const uint2 vi = D ? make_uint2((uint32_t)var * (uint32_t)D, (uint32_t)D)
                                        : __ldg(&P.vinfo[var]);
                     __syncwarp();
-                    apply_flips(P, de, sp, scratch, fm, var, (int)vi.x, (int)(vi.y & kDegMask),
+                    apply_flips<REG>(P, de, sp, scratch, fm, var, (int)vi.x, (int)(vi.y & kDegMask),
                                 s_old, true, lane);
                 }
             }
@@ -1407,7 +1470,7 @@ __device__ __forceinline__ double state_energy(const ProblemDev *PD, const int8_
     return e;
 }
 
-template <bool GIBBS, bool RANDOM_ORDER, bool RESOLVE, int STAGE>
+template <bool GIBBS, bool RANDOM_ORDER, bool RESOLVE, bool REG, int STAGE>
 __device__ __forceinline__ void anneal_read(const ProblemDev *PD, const int8_t *src,
                                             int8_t *dst, double *energy_out,
                                             double *de, int8_t *sp,
@@ -1421,7 +1484,7 @@ __device__ __forceinline__ void anneal_read(const ProblemDev *PD, const int8_t *
             static_assert(STAGE != kStageBand, "the band follows a sequential window");
             typename DeFor<STAGE>::T acc;
             acc.p = de;
-            sweep_random<GIBBS>(P, acc, sp, scratch, ring, rs, lane, touch);
+            sweep_random<GIBBS, REG>(P, acc, sp, scratch, ring, rs, lane, touch);
         } else {
             // A problem whose band does not fit the launch's ring keeps all of
             // its delta energies in the global slot.
@@ -1429,10 +1492,10 @@ __device__ __forceinline__ void anneal_read(const ProblemDev *PD, const int8_t *
                                ? PD->band_w
                                : 0;
             if (RESOLVE && pm1)
-                sweep_resolved<GIBBS, STAGE>(P, de, sp, scratch, ring, rs, lane, band, bw,
+                sweep_resolved<GIBBS, STAGE, REG>(P, de, sp, scratch, ring, rs, lane, band, bw,
                                              PD->band_b);
             else
-                sweep_sequential<GIBBS, STAGE>(P, de, sp, scratch, ring, rs, lane, band, bw,
+                sweep_sequential<GIBBS, STAGE, REG>(P, de, sp, scratch, ring, rs, lane, band, bw,
                                                PD->band_b);
         }
     }

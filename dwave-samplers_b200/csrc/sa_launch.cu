@@ -21,7 +21,7 @@ namespace b200sa {
 
 // K > 0: state in registers, K variables per lane (STAGE is kStageShared, with
 // nothing of the state in the shared region).
-template <bool GIBBS, bool RANDOM_ORDER, bool RESOLVE, int STAGE, int K = 0>
+template <bool GIBBS, bool RANDOM_ORDER, bool RESOLVE, bool REG, int STAGE, int K = 0>
 __device__ __forceinline__ void sa_warp_body(const LaunchArgs &A, int warps_per_cta,
                                              int region_bytes) {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -91,7 +91,7 @@ __device__ __forceinline__ void sa_warp_body(const LaunchArgs &A, int warps_per_
             dense_anneal_read<GIBBS, RANDOM_ORDER, K>(PD, A.states_in + so, A.states_out + so,
                                                       &A.energies[rd], scratch, ring, rs, lane);
         else
-            anneal_read<GIBBS, RANDOM_ORDER, RESOLVE, STAGE>(
+            anneal_read<GIBBS, RANDOM_ORDER, RESOLVE, REG, STAGE>(
                 PD, A.states_in + so, A.states_out + so, &A.energies[rd], de, sp, scratch, ring,
                 rs, lane, touch, band, A.band_cap);
         if (lane == 0) {
@@ -114,61 +114,66 @@ __device__ __forceinline__ void sa_warp_body(const LaunchArgs &A, int warps_per_
     }
 }
 
-template <bool GIBBS, bool RANDOM_ORDER, bool RESOLVE, int STAGE>
+template <bool GIBBS, bool RANDOM_ORDER, bool RESOLVE, bool REG, int STAGE>
 __global__ void __launch_bounds__(kMaxThreadsPerCta, 1)
     sa_warp_kernel(LaunchArgs A, int warps_per_cta, int region_bytes) {
-    sa_warp_body<GIBBS, RANDOM_ORDER, RESOLVE, STAGE>(A, warps_per_cta, region_bytes);
+    sa_warp_body<GIBBS, RANDOM_ORDER, RESOLVE, REG, STAGE>(A, warps_per_cta, region_bytes);
 }
 
-template <bool GIBBS, bool RANDOM_ORDER, bool RESOLVE, int STAGE>
+template <bool GIBBS, bool RANDOM_ORDER, bool RESOLVE, bool REG, int STAGE>
 __global__ void __maxnreg__(kRegs80) sa_warp_kernel_r80(LaunchArgs A, int warps_per_cta,
                                                          int region_bytes) {
-    sa_warp_body<GIBBS, RANDOM_ORDER, RESOLVE, STAGE>(A, warps_per_cta, region_bytes);
+    sa_warp_body<GIBBS, RANDOM_ORDER, RESOLVE, REG, STAGE>(A, warps_per_cta, region_bytes);
 }
 
-template <bool GIBBS, bool RANDOM_ORDER, bool RESOLVE, int STAGE>
+template <bool GIBBS, bool RANDOM_ORDER, bool RESOLVE, bool REG, int STAGE>
 __global__ void __maxnreg__(kRegs64) sa_warp_kernel_r64(LaunchArgs A, int warps_per_cta,
                                                          int region_bytes) {
-    sa_warp_body<GIBBS, RANDOM_ORDER, RESOLVE, STAGE>(A, warps_per_cta, region_bytes);
+    sa_warp_body<GIBBS, RANDOM_ORDER, RESOLVE, REG, STAGE>(A, warps_per_cta, region_bytes);
 }
 
 // State in registers (see dense_reg_class for the budgets).
 template <bool GIBBS, bool RANDOM_ORDER, int K>
 __global__ void __maxnreg__((K <= 2 ? kRegs64 : K <= 4 ? kRegs80 : 128))
     sa_dense_kernel(LaunchArgs A, int warps_per_cta, int region_bytes) {
-    sa_warp_body<GIBBS, RANDOM_ORDER, false, kStageShared, K>(A, warps_per_cta, region_bytes);
+    sa_warp_body<GIBBS, RANDOM_ORDER, false, false, kStageShared, K>(A, warps_per_cta, region_bytes);
 }
 
 using KernelFn = void (*)(LaunchArgs, int, int);
 
 // Kinds in the order of their numbers (bit 0 Gibbs, bit 1 random order,
 // bit 2 in-window resolution); resolution exists for sequential order only.
-#define B200SA_KINDS(name, stage)                                                      \
-    name<false, false, false, stage>, name<true, false, false, stage>,                 \
-        name<false, true, false, stage>, name<true, true, false, stage>,               \
-        name<false, false, true, stage>, name<true, false, true, stage>, nullptr, nullptr
+#define B200SA_KINDS(name, reg, stage)                                                 \
+    name<false, false, false, reg, stage>, name<true, false, false, reg, stage>,       \
+        name<false, true, false, reg, stage>, name<true, true, false, reg, stage>,     \
+        name<false, false, true, reg, stage>, name<true, false, true, reg, stage>,     \
+        nullptr, nullptr
 // The band location exists for sequential order only.
-#define B200SA_SEQ_KINDS(name, stage)                                                  \
-    name<false, false, false, stage>, name<true, false, false, stage>, nullptr, nullptr, \
-        name<false, false, true, stage>, name<true, false, true, stage>, nullptr, nullptr
+#define B200SA_SEQ_KINDS(name, reg, stage)                                             \
+    name<false, false, false, reg, stage>, name<true, false, false, reg, stage>,       \
+        nullptr, nullptr, name<false, false, true, reg, stage>,                        \
+        name<true, false, true, reg, stage>, nullptr, nullptr
 #define B200SA_DENSE_KINDS(K)                                                          \
     {sa_dense_kernel<false, false, K>, sa_dense_kernel<true, false, K>,               \
      sa_dense_kernel<false, true, K>, sa_dense_kernel<true, true, K>}
-#define B200SA_KERNEL_TABLE(name)                                                      \
-    {B200SA_KINDS(name, kStageGlobal), B200SA_KINDS(name, kStageShared),              \
-     B200SA_KINDS(name, kStageSpins), B200SA_SEQ_KINDS(name, kStageBand)}
+#define B200SA_STAGES(name, reg)                                                       \
+    B200SA_KINDS(name, reg, kStageGlobal), B200SA_KINDS(name, reg, kStageShared),      \
+        B200SA_KINDS(name, reg, kStageSpins), B200SA_SEQ_KINDS(name, reg, kStageBand)
+#define B200SA_KERNEL_TABLE(name) {B200SA_STAGES(name, false), B200SA_STAGES(name, true)}
 
 static KernelFn kernel_for(int variant) {
     constexpr int kGeneral = kKindDense;  // kinds below it have a state location
-    constexpr int kPerClass = kNumStages * kGeneral;
+    constexpr int kPerClass = 2 * kNumStages * kGeneral;
     static const KernelFn k128[kPerClass] = B200SA_KERNEL_TABLE(sa_warp_kernel);
     static const KernelFn k80[kPerClass] = B200SA_KERNEL_TABLE(sa_warp_kernel_r80);
     static const KernelFn k64[kPerClass] = B200SA_KERNEL_TABLE(sa_warp_kernel_r64);
     static const KernelFn dense[5][4] = {B200SA_DENSE_KINDS(1), B200SA_DENSE_KINDS(2),
                                          B200SA_DENSE_KINDS(4), B200SA_DENSE_KINDS(8),
                                          B200SA_DENSE_KINDS(kDenseSlots)};
-    if (variant & kKindDense) return dense[variant >> 8][variant & 3];
-    const int idx = ((variant >> 4) & 3) * kGeneral + (variant & (kGeneral - 1));
+    if (variant & kKindDense) return dense[variant_slots(variant)][variant & 3];
+    const int idx = (((variant & kKindRegular) ? kNumStages : 0) + variant_stage(variant)) *
+                        kGeneral +
+                    (variant & (kGeneral - 1));
     switch (variant_reg_class(variant)) {
         case 0: return k128[idx];
         case 1: return k80[idx];

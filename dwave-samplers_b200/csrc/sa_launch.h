@@ -22,7 +22,12 @@ constexpr int kKindGibbs = 1;
 constexpr int kKindRandom = 2;
 constexpr int kKindResolve = 4;
 constexpr int kKindDense = 8;
-constexpr int kNumKinds = 16;
+// Bit 4 equal list lengths (ProblemDev::regular_degree; without bit 3; the
+// two kinds of lists have kernels of their own, each with its path's registers
+// and code alone: uneven batch 93.6 -> 88.6 ms, 50 reads of a sparse n = 20011
+// problem 26.1 -> 23.6, n = 1000, 1000 reads 4.7 -> 4.2).
+constexpr int kKindRegular = 16;
+constexpr int kNumKinds = 32;
 
 // Kernels with the state in registers: 1, 2, 4, 8 or kDenseSlots variables per
 // lane by the launch's largest n, one register budget each.
@@ -31,15 +36,17 @@ inline int dense_slots(int max_n) {
 }
 inline int dense_reg_class(int max_n) { return max_n <= 64 ? 2 : max_n <= 128 ? 1 : 0; }
 
-// Kernel variant: bits 0-3 kind, bits 4-5 state location (kStageGlobal,
-// kStageShared, kStageSpins, kStageBand), bits 6-7 register class (0: 128, 1:
-// 80, 2: 64 registers), bits 8-10 dense_slots of kinds with the state in
+// Kernel variant: bits 0-4 kind, bits 5-6 state location (kStageGlobal,
+// kStageShared, kStageSpins, kStageBand), bits 7-8 register class (0: 128, 1:
+// 80, 2: 64 registers), bits 9-11 dense_slots of kinds with the state in
 // registers.
 inline int kernel_variant(int kind, int stage, int reg_class = 0, int max_n = 0) {
-    return (kind & (kNumKinds - 1)) | (stage << 4) | (reg_class << 6) |
-           ((kind & kKindDense) ? dense_slots(max_n) << 8 : 0);
+    return (kind & (kNumKinds - 1)) | (stage << 5) | (reg_class << 7) |
+           ((kind & kKindDense) ? dense_slots(max_n) << 9 : 0);
 }
-inline int variant_reg_class(int variant) { return (variant >> 6) & 3; }
+inline int variant_stage(int variant) { return (variant >> 5) & 3; }
+inline int variant_reg_class(int variant) { return (variant >> 7) & 3; }
+inline int variant_slots(int variant) { return variant >> 9; }
 
 // Bytes of the touch bitmap of a launch (random order outside registers).
 inline int kind_touch_bytes(int kind, int max_n) {

@@ -205,7 +205,8 @@ B200SA_API int b200sa_plan_set_weights_device(b200sa_plan plan, const double *d_
 typedef struct {
     int32_t bucket;
     int32_t kind;           /* bit 0 Gibbs, bit 1 random order, bit 2 in-window
-                             * resolution, bit 3 state in registers */
+                             * resolution, bit 3 state in registers, bit 4
+                             * equal list lengths */
     int32_t max_n;
     int64_t items;          /* reads in the bucket */
     int32_t staging;        /* state: 0 global slot (L2), 1 shared memory, 2 spins in
@@ -236,7 +237,8 @@ B200SA_API int b200sa_plan_autotune(b200sa_plan plan, const char *cache_path, in
 typedef struct {
     int32_t bucket;
     int32_t kind;           /* bit 0 Gibbs, bit 1 random order, bit 2 in-window
-                             * resolution, bit 3 state in registers */
+                             * resolution, bit 3 state in registers, bit 4
+                             * equal list lengths */
     int32_t max_n;
     int64_t reads;
     int64_t attempts;
