@@ -785,8 +785,8 @@ struct Choice {
 
     // Per beta: beta log2(e), the factor of d.
     static __device__ __forceinline__ float scale(double beta) {
-        return beta > 1e-30 && beta < 1e30 ? (float)(beta * (double)kLog2e)
-                                           : __int_as_float(0x7fffffff);
+        return beta == 0.0 || (beta > 1e-30 && beta < 1e30) ? (float)(beta * (double)kLog2e)
+                                                            : __int_as_float(0x7fffffff);
     }
     __device__ __forceinline__ void look(double d, float scale, double thr, bool act) {
         const float inf = __int_as_float(0x7f800000);
