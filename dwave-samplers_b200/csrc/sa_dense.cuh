@@ -322,7 +322,7 @@ __device__ __forceinline__ void dense_anneal_read(const ProblemDev *PD, const in
     __syncwarp();
     for (int v = (int)lane; v < n; v += 32) dst[v] = sp[v];
     __syncwarp();
-    const double e = state_energy(PD, sp, lane);
+    const double e = state_energy(PD, sp, nullptr, lane);
     if (lane == 0) *energy_out = e;
     __syncwarp();
 }

@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1)
             ++steps;
         }
         __syncwarp();
-        const double e = state_energy(PD, sp, lane);  // descent.cpp:75-93
+        const double e = state_energy(PD, sp, scratch, lane);  // descent.cpp:75-93
         for (int v = lane; v < n; v += 32) A.states_out[so + v] = sp[v];
         if (lane == 0) {
             A.energies[PD->read_offset + r] = e;
