@@ -106,10 +106,11 @@ extern "C" int b200sa_path_anneal(
     const int cap_props = break_capacity ? break_capacity : auto_capacity(hd_field, num_betas);
     const int cap_breaks = std::max(cap_props, (max_in + 3) & ~3);
     // Single-qubit updates run on a warp per sample while a CTA's warps fit in
-    // shared memory; chain updates, very large capacities and break lists out
-    // of order on one thread per sample.
+    // shared memory; chain updates, very large capacities, break lists out of
+    // order and more than kPimcThreadSamples samples on one thread per sample.
     const int64_t warp_bytes = pimc_warp_bytes(cap_props, cap_breaks);
-    const bool warp = !chain && ordered && warp_bytes <= 48 * 1024;
+    const bool warp = !chain && ordered && warp_bytes <= 48 * 1024 &&
+                      (num_seeds == 1 || num_samples <= kPimcThreadSamples);
     const int Q = chain ? qubits_per_chain : 1;
     const int64_t C = (int64_t)cap_props + cap_breaks;
     // props, itf [Q][C], sv [Q * C], off [Q + 1], lab [Q * C], parent [Q * C], pair [2C]

@@ -252,6 +252,13 @@ constexpr int kPimcSlices = 65536;  // numTrotterSlices, localPIMC.h:88
 // Warps per CTA of the warp-per-sample kernel at most, and its shared memory
 // per sample: mt19937 state, scratch (PimcWarpScratch).
 constexpr int kPimcMaxWarps = 4;
+// Above this many samples single-qubit updates run one thread per sample: the
+// threads then fill the chip, while a warp per sample already issues at its
+// limit and its time grows with the samples.  n = 512, 16 steps, field 5 ->
+// 0.05, kernel time of a warp and of a thread per sample: 151 and 249 ms with
+// 16384 samples, 288 and 315 with 32768, 566 and 497 with 65536; lines through
+// these cross near 41000.
+constexpr int64_t kPimcThreadSamples = 40960;
 inline int64_t pimc_warp_bytes(int64_t cap_props, int64_t cap_breaks) {
     const int64_t cap = cap_props + cap_breaks;
     return (4 * kMtWords + 32 * (8 + 4 + 4) + 8 * cap + cap + 15) & ~int64_t(15);
