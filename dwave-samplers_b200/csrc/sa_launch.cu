@@ -9,6 +9,9 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <mutex>
+#include <set>
+#include <utility>
 
 #include "sa_kernel.cuh"
 #include "sa_launch.h"
@@ -267,12 +270,39 @@ cudaError_t upload_jump_table(const uint32_t table[][4], cudaStream_t stream) {
                                    cudaMemcpyHostToDevice, stream);
 }
 
+// Lets kernel `k` be launched with all of the shared memory a CTA may have.  The
+// limit belongs to the function, so host threads share it: it is raised once per
+// function and device and never lowered, and a launch or an occupancy query of
+// one thread cannot take it below what another one is about to launch with.
+static cudaError_t open_smem(const void *k) {
+    static std::mutex mutex;
+    static std::set<std::pair<int, const void *>> open;
+    int device = 0, most = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mutex);
+    if (open.count({device, k})) return cudaSuccess;
+    cudaFuncAttributes attr;
+    if ((e = cudaFuncGetAttributes(&attr, k)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device)) !=
+        cudaSuccess)
+        return e;
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             most - (int)attr.sharedSizeBytes);
+    if (e == cudaSuccess) open.insert({device, k});
+    return e;
+}
+template <class... ARGS>
+static cudaError_t open_smem(void (*k)(ARGS...)) {
+    return open_smem(reinterpret_cast<const void *>(k));
+}
+
 cudaError_t launch_sa(int variant, const LaunchArgs &args, int grid, int warps_per_cta,
                       int region_bytes, cudaStream_t stream) {
     const KernelFn k = kernel_for(variant);
     if (!k) return cudaErrorInvalidValue;
     const size_t smem = (size_t)warps_per_cta * (size_t)region_bytes;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = open_smem(k);
     if (e != cudaSuccess) return e;
     k<<<grid, warps_per_cta * 32, smem, stream>>>(args, warps_per_cta, region_bytes);
     return cudaGetLastError();
@@ -282,7 +312,7 @@ cudaError_t kernel_occupancy(int variant, int warps_per_cta, int region_bytes, i
     const KernelFn k = kernel_for(variant);
     if (!k) return cudaErrorInvalidValue;
     const size_t smem = (size_t)warps_per_cta * (size_t)region_bytes;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = open_smem(k);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, k, warps_per_cta * 32, smem);
 }
@@ -298,7 +328,7 @@ cudaError_t launch_sd(bool sparse, bool smem, const SdArgs &args, int grid, int 
                       int region_bytes, cudaStream_t stream) {
     const SdKernel k = sd_kernel_for(sparse, smem);
     const size_t bytes = (size_t)args.table_bytes + (size_t)warps_per_cta * (size_t)region_bytes;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    cudaError_t e = open_smem(k);
     if (e != cudaSuccess) return e;
     k<<<grid, warps_per_cta * 32, bytes, stream>>>(args, warps_per_cta, region_bytes);
     return cudaGetLastError();
@@ -308,7 +338,7 @@ cudaError_t sd_occupancy(bool sparse, bool smem, int warps_per_cta, int region_b
                          int table_bytes, int *ctas_per_sm) {
     const SdKernel k = sd_kernel_for(sparse, smem);
     const size_t bytes = (size_t)table_bytes + (size_t)warps_per_cta * (size_t)region_bytes;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    cudaError_t e = open_smem(k);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, k, warps_per_cta * 32, bytes);
 }
@@ -334,7 +364,7 @@ static RmcKernel rmc_kernel_for(bool random_order, int proposal, int stage) {
 static cudaError_t rmc_smem(RmcKernel k, int warps_per_cta, int64_t region_bytes, size_t &smem) {
     if (!k) return cudaErrorInvalidValue;
     smem = (size_t)kRmcTableBytes + (size_t)warps_per_cta * (size_t)region_bytes;
-    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return open_smem(k);
 }
 
 cudaError_t launch_rmc(bool random_order, int proposal, int stage, const RmcArgs &args, int grid,
@@ -378,8 +408,7 @@ cudaError_t launch_pimc(bool chain_update, const PimcArgs &args, int grid, int b
 cudaError_t launch_pimc_warp(const PimcArgs &args, int grid, int warps_per_cta, int warp_bytes,
                              cudaStream_t stream) {
     const size_t smem = (size_t)warps_per_cta * (size_t)warp_bytes;
-    const cudaError_t e = cudaFuncSetAttribute(
-        pimc_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = open_smem(pimc_warp_kernel);
     if (e != cudaSuccess) return e;
     pimc_warp_kernel<<<grid, warps_per_cta * 32, smem, stream>>>(args, warp_bytes);
     return cudaGetLastError();
