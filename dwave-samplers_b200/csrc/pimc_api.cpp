@@ -149,6 +149,7 @@ extern "C" int b200sa_path_anneal(
     cudaDeviceProp prop;
     int rc = select_device(device, prop, err, errlen);
     if (rc) return rc;
+    IdleScope scope;
     DevArray<uint2> dvinfo;
     DevArray<int32_t> dcol, dcu, dcv, dcnt, dbrk, dscr_i, dflag;
     DevArray<double> dw, dh, dcw, dhp, dhd, den, dscr_d;
@@ -253,14 +254,16 @@ extern "C" int b200sa_path_anneal(
         const int grid = shared ? 1 : (int)((R + block - 1) / block);
         B200SA_CUDA(launch_pimc(chain, a, grid, block, nullptr));
     }
-    B200SA_CUDA(cudaDeviceSynchronize());
+    B200SA_CUDA(cudaStreamSynchronize(nullptr));
     int32_t overflow = 0;
     B200SA_CUDA(cudaMemcpy(&overflow, dflag.ptr, sizeof(overflow), cudaMemcpyDeviceToHost));
-    if (overflow)
+    if (overflow) {
+        IdleScope::done();
         return set_err(err, errlen, B200SA_ERANGE,
                        "a break list or the break proposals of one update exceeded the capacity " +
                            std::to_string(cap_props) +
                            "; call again with a larger break_capacity");
+    }
     B200SA_CUDA(cudaMemcpy(states, dst.ptr, n * R, cudaMemcpyDeviceToHost));
     B200SA_CUDA(cudaMemcpy(energies, den.ptr, 8 * R, cudaMemcpyDeviceToHost));
     unsigned long long near = 0;
@@ -293,5 +296,6 @@ extern "C" int b200sa_path_anneal(
             start += total;
         }
     }
+    IdleScope::done();
     return num_samples;
 }

@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "b200sa.h"
+#include "pool.h"
 #include "sa_launch.h"
 #include "sa_types.h"
 
@@ -49,22 +50,6 @@ struct DeviceGuard {
 // Makes `device` current and returns its properties (queried once per device
 // and process: a query takes 2.5 ms).
 int select_device(int device, cudaDeviceProp &prop, char *err, size_t errlen);
-
-// Device memory and non-blocking streams of the current device, reused from
-// call to call: a call's buffers and stream otherwise cost it about 20
-// microseconds each to make and as many to free (0.7 ms for 8 MB, 0.15 to 0.2
-// ms for a stream).  Freed blocks of at most kPoolBlock bytes are kept, up to
-// kPoolBytes in all per device, and go back to the driver when an allocation
-// fails; streams likewise up to kPoolStreams.  Every function may be called
-// from any thread.  pool_free waits for the device, as cudaFree does, so a
-// block is never handed out while work in flight may use it.
-constexpr size_t kPoolBlock = size_t(64) << 20;
-constexpr size_t kPoolBytes = size_t(256) << 20;
-constexpr size_t kPoolStreams = 16;
-cudaError_t pool_alloc(void **ptr, size_t bytes);
-void pool_free(void *ptr, size_t bytes, int device);
-cudaError_t pool_stream(cudaStream_t *stream);
-void pool_stream_free(cudaStream_t stream, int device);  // with no work in flight
 
 template <typename T>
 struct DevArray {
@@ -255,6 +240,9 @@ int shape_for(b200sa_plan_s *P, int kind, int32_t max_n_here, int64_t items, boo
               LaunchShape &out, char *err, size_t errlen, const TuneChoice *choice = nullptr,
               int band_w_here = 0);
 int ensure_scratch(b200sa_plan_s *P, int64_t slots, int64_t stride, char *err, size_t errlen);
+// Destroys the plan of one call at its end; a call that has waited for its work
+// (IdleScope) does not wait for the device again.
+void release_plan(b200sa_plan plan);
 LaunchArgs base_args(b200sa_plan_s *P, const int8_t *in, int8_t *out, double *en,
                      const uint64_t *seeds);
 int launch_items(b200sa_plan_s *P, LaunchArgs a, int kind, const int64_t *items, int64_t count,

@@ -81,6 +81,7 @@ extern "C" int b200sa_rotor_anneal(int32_t num_vars, const double *h, int64_t nu
                            ? 1 + (num_betas - 1) / schedule_sample_interval
                            : 0;
     const size_t n = (size_t)num_vars, R = (size_t)num_samples, m = (size_t)num_couplers;
+    IdleScope scope;
     DevArray<uint2> dvinfo;
     DevArray<int32_t> dcol, dcu, dcv;
     DevArray<double> dw, dh, dtf, dcw, dhp, dhd, dde, den, dtab;
@@ -215,7 +216,7 @@ extern "C" int b200sa_rotor_anneal(int32_t num_vars, const double *h, int64_t nu
         }
         B200SA_CUDA(launch_rmc(random, proposal, stage, a, grid, width, nullptr));
     }
-    B200SA_CUDA(cudaDeviceSynchronize());
+    B200SA_CUDA(cudaStreamSynchronize(nullptr));
     B200SA_CUDA(cudaMemcpy(states, drows.ptr, n * R, cudaMemcpyDeviceToHost));
     B200SA_CUDA(cudaMemcpy(energies, den.ptr, 8 * R, cudaMemcpyDeviceToHost));
     unsigned long long near = 0;
@@ -234,5 +235,6 @@ extern "C" int b200sa_rotor_anneal(int32_t num_vars, const double *h, int64_t nu
             std::memcpy(statistics + r * stride, blocks.data() + r * (size_t)points * n,
                         (size_t)points * n);
     }
+    IdleScope::done();
     return num_samples;
 }

@@ -62,107 +62,6 @@ int select_device(int device, cudaDeviceProp &prop, char *err, size_t errlen) {
 }
 
 
-namespace {
-
-// What pool_free and pool_stream_free keep, per device.  Never destroyed: the
-// driver takes everything back when the process ends.
-struct DevicePool {
-    std::map<size_t, std::vector<void *>> blocks;  // by size class
-    size_t bytes = 0;
-    std::vector<cudaStream_t> streams;
-};
-std::mutex g_pool_mutex;
-std::map<int, DevicePool> &device_pools() {
-    static auto *pools = new std::map<int, DevicePool>();
-    return *pools;
-}
-
-size_t pool_class(size_t bytes) {
-    size_t c = 512;
-    while (c < bytes) c <<= 1;
-    return c;
-}
-
-}  // namespace
-
-cudaError_t pool_alloc(void **ptr, size_t bytes) {
-    int device = 0;
-    cudaError_t e = cudaGetDevice(&device);
-    if (e != cudaSuccess) return e;
-    const size_t size = bytes <= kPoolBlock ? pool_class(bytes) : bytes;
-    if (bytes <= kPoolBlock) {
-        std::lock_guard<std::mutex> lock(g_pool_mutex);
-        DevicePool &pool = device_pools()[device];
-        auto it = pool.blocks.find(size);
-        if (it != pool.blocks.end() && !it->second.empty()) {
-            *ptr = it->second.back();
-            it->second.pop_back();
-            pool.bytes -= size;
-            return cudaSuccess;
-        }
-    }
-    e = cudaMalloc(ptr, size);
-    if (e != cudaErrorMemoryAllocation) return e;
-    cudaGetLastError();
-    std::vector<void *> back;  // give everything back and try once more
-    {
-        std::lock_guard<std::mutex> lock(g_pool_mutex);
-        DevicePool &pool = device_pools()[device];
-        for (auto &b : pool.blocks) back.insert(back.end(), b.second.begin(), b.second.end());
-        pool.blocks.clear();
-        pool.bytes = 0;
-    }
-    for (void *b : back) cudaFree(b);
-    return cudaMalloc(ptr, bytes <= kPoolBlock ? size : bytes);
-}
-
-void pool_free(void *ptr, size_t bytes, int device) {
-    int current = 0;
-    if (cudaGetDevice(&current) != cudaSuccess) current = device;
-    if (current != device) cudaSetDevice(device);
-    const size_t size = bytes <= kPoolBlock ? pool_class(bytes) : 0;
-    bool kept = false;
-    if (size && cudaDeviceSynchronize() == cudaSuccess) {
-        std::lock_guard<std::mutex> lock(g_pool_mutex);
-        DevicePool &pool = device_pools()[device];
-        if (pool.bytes + size <= kPoolBytes) {
-            pool.blocks[size].push_back(ptr);
-            pool.bytes += size;
-            kept = true;
-        }
-    }
-    if (!kept) cudaFree(ptr);
-    if (current != device) cudaSetDevice(current);
-}
-
-cudaError_t pool_stream(cudaStream_t *stream) {
-    int device = 0;
-    const cudaError_t e = cudaGetDevice(&device);
-    if (e != cudaSuccess) return e;
-    {
-        std::lock_guard<std::mutex> lock(g_pool_mutex);
-        std::vector<cudaStream_t> &free = device_pools()[device].streams;
-        if (!free.empty()) {
-            *stream = free.back();
-            free.pop_back();
-            return cudaSuccess;
-        }
-    }
-    return cudaStreamCreateWithFlags(stream, cudaStreamNonBlocking);
-}
-
-void pool_stream_free(cudaStream_t stream, int device) {
-    if (cudaStreamSynchronize(stream) == cudaSuccess) {
-        std::lock_guard<std::mutex> lock(g_pool_mutex);
-        std::vector<cudaStream_t> &free = device_pools()[device].streams;
-        if (free.size() < kPoolStreams) {
-            free.push_back(stream);
-            return;
-        }
-    }
-    cudaStreamDestroy(stream);
-}
-
 // In-window resolution of the sequential sweep is on unless the environment
 // sets B200SA_RESOLVE=0 (results are identical either way; for A/B timing).
 bool resolve_allowed() {
@@ -379,7 +278,7 @@ int ensure_scratch(b200sa_plan_s *P, int64_t slots, int64_t stride, char *err,
     stride = std::max(stride, P->scratch_stride);
     // The old slots may still be in use by an enqueued run, and a captured
     // graph holds their addresses.
-    B200SA_CUDA(cudaDeviceSynchronize());
+    if (P->scratch_slots || P->graph_exec) B200SA_CUDA(cudaDeviceSynchronize());
     if (P->graph_exec) {
         cudaGraphExecDestroy(P->graph_exec);
         P->graph_exec = nullptr;
@@ -389,6 +288,16 @@ int ensure_scratch(b200sa_plan_s *P, int64_t slots, int64_t stride, char *err,
     P->scratch_slots = slots;
     P->scratch_stride = stride;
     return B200SA_OK;
+}
+
+void release_plan(b200sa_plan plan) {
+    if (!IdleScope::idle()) {
+        b200sa_plan_destroy(plan);
+        return;
+    }
+    DeviceGuard guard;
+    cudaSetDevice(plan->device);
+    delete plan;
 }
 
 LaunchArgs base_args(b200sa_plan_s *P, const int8_t *in, int8_t *out, double *en,
@@ -874,7 +783,11 @@ int b200sa_plan_destroy(b200sa_plan plan) {
     if (!plan) return B200SA_OK;
     DeviceGuard guard;
     cudaSetDevice(plan->device);
-    cudaDeviceSynchronize();
+    IdleScope scope;
+    if (cudaDeviceSynchronize() == cudaSuccess)
+        IdleScope::done();
+    else
+        cudaGetLastError();
     delete plan;
     return B200SA_OK;
 }
@@ -959,10 +872,11 @@ int b200sa_sample_batch(const b200sa_problem *problems, int32_t num_problems, in
             return set_err(err, errlen, B200SA_EINVAL,
                            "problem " + std::to_string(i) + ": energies is NULL");
     }
+    IdleScope scope;
     b200sa_plan plan = nullptr;
     int rc = b200sa_plan_create(problems, num_problems, device, &plan, err, errlen);
     if (rc) return rc;
-    std::unique_ptr<b200sa_plan_s, int (*)(b200sa_plan)> hold(plan, b200sa_plan_destroy);
+    std::unique_ptr<b200sa_plan_s, void (*)(b200sa_plan)> hold(plan, release_plan);
     const char *cache = std::getenv("B200SA_TUNE_CACHE");
     if (cache && *cache && mode != B200SA_MODE_PLAIN) {
         rc = b200sa_plan_autotune(plan, cache, 0, nullptr, 0, err, errlen);
@@ -994,6 +908,7 @@ int b200sa_sample_batch(const b200sa_problem *problems, int32_t num_problems, in
                                         cudaMemcpyDeviceToHost, plan->stream));
     }
     B200SA_CUDA(cudaStreamSynchronize(plan->stream));
+    IdleScope::done();
     return (int)std::min<int64_t>(plan->total_reads, INT32_MAX);
 }
 
@@ -1052,10 +967,11 @@ int b200sa_sample(int32_t num_vars, const double *h, int64_t num_couplers,
         if (stats) stats->reads = num_reads;
         return num_reads;
     }
+    IdleScope scope;
     b200sa_plan plan = nullptr;
     int rc = b200sa_plan_create(&q, 1, device, &plan, err, errlen);
     if (rc) return rc;
-    std::unique_ptr<b200sa_plan_s, int (*)(b200sa_plan)> hold(plan, b200sa_plan_destroy);
+    std::unique_ptr<b200sa_plan_s, void (*)(b200sa_plan)> hold(plan, release_plan);
     DeviceGuard guard;
     B200SA_CUDA(cudaSetDevice(plan->device));
     const size_t n = (size_t)num_vars;
@@ -1129,6 +1045,7 @@ int b200sa_sample(int32_t num_vars, const double *h, int64_t num_couplers,
         if (rc) return rc;
         stats->kernel_ms = total_ms;
     }
+    IdleScope::done();
     return done;
 }
 

@@ -50,10 +50,11 @@ extern "C" int b200sa_steepest_descent(int32_t num_vars, const double *h, int64_
     q.seeds = seeds.data();
     q.varorder = B200SA_SEQUENTIAL;
     q.proposal = B200SA_METROPOLIS;
+    IdleScope scope;
     b200sa_plan plan = nullptr;
     int rc = b200sa_plan_create(&q, 1, device, &plan, err, errlen);
     if (rc) return rc;
-    std::unique_ptr<b200sa_plan_s, int (*)(b200sa_plan)> hold(plan, b200sa_plan_destroy);
+    std::unique_ptr<b200sa_plan_s, void (*)(b200sa_plan)> hold(plan, release_plan);
     DeviceGuard guard;
     B200SA_CUDA(cudaSetDevice(plan->device));
     const bool sparse = large_sparse_opt != 0;
@@ -146,6 +147,7 @@ extern "C" int b200sa_steepest_descent(int32_t num_vars, const double *h, int64_
     B200SA_CUDA(cudaMemcpyAsync(&capped, counters.ptr + 1, sizeof(capped),
                                 cudaMemcpyDeviceToHost, st));
     B200SA_CUDA(cudaStreamSynchronize(st));
+    IdleScope::done();
     if (capped)
         return set_err(err, errlen, B200SA_ETIMEOUT,
                        std::to_string(capped) + " sample(s) stopped after max_steps = " +
