@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import argparse
 import glob
+import hashlib
 import os
 import shutil
 import subprocess
@@ -45,11 +46,19 @@ def stale() -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def digest() -> str:
+    """Of the sources: part of the tuning cache's keys."""
+    h = hashlib.sha256()
+    for f in sorted(glob.glob(os.path.join(CSRC, "*"))):
+        h.update(open(f, "rb").read())
+    return h.hexdigest()[:12]
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not stale():
         return OUT
     tmp = OUT + ".tmp"
-    cmd = [nvcc(), *ARCH, *FLAGS, "-shared", "-cudart", "static", "-I", INCLUDE, "-I", CSRC,
+    cmd = [nvcc(), *ARCH, *FLAGS, f'-DB200SA_SOURCES="{digest()}"', "-shared", "-cudart", "static", "-I", INCLUDE, "-I", CSRC,
            *sources(), "-o", tmp]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:

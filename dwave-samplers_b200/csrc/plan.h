@@ -143,6 +143,7 @@ struct LaunchShape {
     int variant;
     int touch_bytes;   // random order: the touch bitmap inside the region
     int band_cap;      // kStageBand: slots of the delta-energy band
+    bool tuned;        // from the tuned choice, not from the occupancy rule
 };
 
 // Arena byte offsets of one packed problem.

@@ -68,6 +68,12 @@ namespace {
 constexpr int kTuneBetas = 8;     // betas per sampled schedule
 constexpr int kTuneWarpsPerSm = 64;  // sample reads per SM: two waves at 32 warps per SM
 
+// The sources' digest (build.py): entries of other kernels or layouts are not
+// taken.
+#ifndef B200SA_SOURCES
+#define B200SA_SOURCES "unknown"
+#endif
+
 std::string tune_key(const b200sa_plan_s *P, int kind, int max_n, int mean_degree) {
     std::string name = P->prop.name;
     for (char &c : name)
@@ -75,7 +81,7 @@ std::string tune_key(const b200sa_plan_s *P, int kind, int max_n, int mean_degre
     const int n_bin = (max_n + 63) / 64 * 64;
     std::ostringstream k;
     k << "gpu=" << name << ";sms=" << P->prop.multiProcessorCount << ";lib=" << b200sa_version()
-      << ";kind=" << (kind & ~kKindRegular) << ";n=" << n_bin << ";deg=" << mean_degree;
+      << ";src=" << B200SA_SOURCES << ";kind=" << kind << ";n=" << n_bin << ";deg=" << mean_degree;
     std::string s = k.str();
     for (char &c : s)
         if (c == ' ') c = '_';
@@ -455,8 +461,13 @@ int b200sa_plan_autotune(b200sa_plan plan, const char *cache_path, int32_t flags
         bool cached = false;
         auto hit = cache.find(key);
         if (!(flags & B200SA_TUNE_FORCE) && hit != cache.end()) {
+            LaunchShape s{};  // an entry that does not fit here is measured anew
+            rc = shape_for(plan, kind, max_n, cnt, true, s, err, errlen, &hit->second, band_w);
+            if (rc) return rc;
+            cached = s.tuned;
+        }
+        if (cached) {
             best = hit->second;
-            cached = true;
         } else {
             // Candidates: per register budget and staging, every
             // warps-per-CTA whose resident warps per SM come within 7/8 of

@@ -193,6 +193,7 @@ int shape_for(b200sa_plan_s *P, int kind, int32_t max_n_here, int64_t items, boo
     const int region = region_bytes_for_stage(stage, cap, band_cap) + tb;
     out.touch_bytes = tb;
     out.band_cap = band_cap;
+    out.tuned = false;
     // (80 registers only where shared memory leaves room for more than the
     // 16 warps per SM of the 128-register kernel.)
     const bool more_warps =
@@ -208,12 +209,15 @@ int shape_for(b200sa_plan_s *P, int kind, int32_t max_n_here, int64_t items, boo
         // The autotuner's measured configuration (a persistent launch takes
         // items from its queue; a plain one strides over them statically).
         const int w = choice->warps_per_cta;
-        if (w < 1 || w > kMaxThreadsPerCta / 32 || (int64_t)w * region > smem_blk)
-            return set_err(err, errlen, B200SA_EINVAL, "tuned shape does not fit");
         int ctas = 0;
-        int rc = occupancy(P, variant, w, region, &ctas, err, errlen);
-        if (rc) return rc;
-        if (ctas < 1) return set_err(err, errlen, B200SA_ECUDA, "tuned shape does not fit on an SM");
+        if (w >= 1 && w <= kMaxThreadsPerCta / 32 && (int64_t)w * region <= smem_blk) {
+            int rc = occupancy(P, variant, w, region, &ctas, err, errlen);
+            if (rc) return rc;
+        }
+        if (ctas < 1)  // tuned on a smaller problem or band of the same key
+            return shape_for(P, kind, max_n_here, items, persistent, out, err, errlen, nullptr,
+                             band_w_here);
+        out.tuned = true;
         if (choice->ctas_per_sm > 0) ctas = std::min(ctas, choice->ctas_per_sm);
         int wl = w;
         if (!persistent) {

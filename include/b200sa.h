@@ -198,8 +198,9 @@ B200SA_API int b200sa_plan_set_weights_device(b200sa_plan plan, const double *d_
  * schedule) and keeps the fastest for the plan's persistent and graph runs.
  * Every configuration computes the same results; only speed changes.  The
  * choices are cached in the text file `cache_path` (NULL: no file), keyed by
- * GPU, library version, kind, size and mean degree, and reused unless flags
- * has B200SA_TUNE_FORCE.  Writes up to report_cap entries and returns the
+ * GPU, library version and sources, kind, size and mean degree, and reused
+ * unless flags has B200SA_TUNE_FORCE or an entry does not fit the bucket; a
+ * run whose problems a choice does not fit takes the untuned shape.  Writes up to report_cap entries and returns the
  * number of non-empty buckets, or a negative error. */
 #define B200SA_TUNE_FORCE 1
 typedef struct {
