@@ -55,13 +55,14 @@ template <typename T>
 struct DevArray {
     T *ptr = nullptr;
     size_t count = 0;
-    int device = 0;  // of the allocation
+    size_t size = 0;  // bytes of the block
+    int device = 0;   // of the allocation
     DevArray() = default;
     DevArray(const DevArray &) = delete;
     DevArray &operator=(const DevArray &) = delete;
     ~DevArray() { release(); }
     void release() {
-        if (ptr) pool_free(ptr, count * sizeof(T), device);
+        if (ptr) pool_free(ptr, size, device);
         ptr = nullptr;
         count = 0;
     }
@@ -69,7 +70,7 @@ struct DevArray {
         release();
         if (n == 0) return cudaSuccess;
         cudaError_t e = cudaGetDevice(&device);
-        if (e == cudaSuccess) e = pool_alloc(reinterpret_cast<void **>(&ptr), n * sizeof(T));
+        if (e == cudaSuccess) e = pool_alloc(reinterpret_cast<void **>(&ptr), n * sizeof(T), &size);
         if (e == cudaSuccess) count = n;
         return e;
     }

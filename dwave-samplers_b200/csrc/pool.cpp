@@ -1,6 +1,8 @@
 // Device memory and streams reused from call to call (pool.h).
 #include "pool.h"
 
+#include <algorithm>
+#include <list>
 #include <map>
 #include <mutex>
 #include <vector>
@@ -14,8 +16,12 @@ namespace {
 
 // What pool_free and pool_stream_free keep, per device.  Never destroyed: the
 // driver takes everything back when the process ends.
+struct Block {
+    void *ptr;
+    size_t size;
+};
 struct DevicePool {
-    std::map<size_t, std::vector<void *>> blocks;  // by size class
+    std::list<Block> blocks;  // oldest first
     size_t bytes = 0;
     std::vector<cudaStream_t> streams;
 };
@@ -25,60 +31,64 @@ std::map<int, DevicePool> &device_pools() {
     return *pools;
 }
 
-size_t pool_class(size_t bytes) {
-    size_t c = 512;
-    while (c < bytes) c <<= 1;
-    return c;
-}
-
 }  // namespace
 
-cudaError_t pool_alloc(void **ptr, size_t bytes) {
+cudaError_t pool_alloc(void **ptr, size_t bytes, size_t *size) {
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
-    const size_t size = bytes <= kPoolBlock ? pool_class(bytes) : bytes;
+    bytes = (bytes + 511) & ~size_t(511);
     if (bytes <= kPoolBlock) {
+        const size_t most = bytes + std::max(bytes / 8, kPoolSlack);
         std::lock_guard<std::mutex> lock(g_pool_mutex);
         DevicePool &pool = device_pools()[device];
-        auto it = pool.blocks.find(size);
-        if (it != pool.blocks.end() && !it->second.empty()) {
-            *ptr = it->second.back();
-            it->second.pop_back();
-            pool.bytes -= size;
+        auto best = pool.blocks.end();
+        for (auto it = pool.blocks.begin(); it != pool.blocks.end(); ++it)
+            if (it->size >= bytes && it->size <= most &&
+                (best == pool.blocks.end() || it->size < best->size))
+                best = it;
+        if (best != pool.blocks.end()) {
+            *ptr = best->ptr;
+            *size = best->size;
+            pool.bytes -= best->size;
+            pool.blocks.erase(best);
             return cudaSuccess;
         }
     }
-    e = cudaMalloc(ptr, size);
+    *size = bytes;
+    e = cudaMalloc(ptr, bytes);
     if (e != cudaErrorMemoryAllocation) return e;
     cudaGetLastError();
-    std::vector<void *> back;  // give everything back and try once more
+    std::list<Block> back;  // give everything back and try once more
     {
         std::lock_guard<std::mutex> lock(g_pool_mutex);
         DevicePool &pool = device_pools()[device];
-        for (auto &b : pool.blocks) back.insert(back.end(), b.second.begin(), b.second.end());
-        pool.blocks.clear();
+        back.swap(pool.blocks);
         pool.bytes = 0;
     }
-    for (void *b : back) cudaFree(b);
-    return cudaMalloc(ptr, bytes <= kPoolBlock ? size : bytes);
+    for (const Block &b : back) cudaFree(b.ptr);
+    return cudaMalloc(ptr, bytes);
 }
 
-void pool_free(void *ptr, size_t bytes, int device) {
-    const size_t size = bytes <= kPoolBlock ? pool_class(bytes) : 0;
-    if (size && IdleScope::idle()) {
+void pool_free(void *ptr, size_t size, int device) {
+    std::list<Block> back;
+    if (size <= kPoolBlock && IdleScope::idle()) {
         std::lock_guard<std::mutex> lock(g_pool_mutex);
         DevicePool &pool = device_pools()[device];
-        if (pool.bytes + size <= kPoolBytes) {
-            pool.blocks[size].push_back(ptr);
-            pool.bytes += size;
-            return;
+        pool.blocks.push_back({ptr, size});
+        pool.bytes += size;
+        while (pool.bytes > kPoolBytes) {
+            pool.bytes -= pool.blocks.front().size;
+            back.splice(back.end(), pool.blocks, pool.blocks.begin());
         }
+    } else {
+        back.push_back({ptr, size});
     }
+    if (back.empty()) return;
     int current = 0;
     if (cudaGetDevice(&current) != cudaSuccess) current = device;
     if (current != device) cudaSetDevice(device);
-    cudaFree(ptr);
+    for (const Block &b : back) cudaFree(b.ptr);
     if (current != device) cudaSetDevice(current);
 }
 

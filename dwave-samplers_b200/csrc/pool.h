@@ -11,16 +11,21 @@ namespace host {
 // call to call: a call's buffers and stream otherwise cost it about 20
 // microseconds each to make and as many to free (0.7 ms for 8 MB, 0.15 to 0.2
 // ms for a stream).  Freed blocks of at most kPoolBlock bytes are kept, up to
-// kPoolBytes in all per device, and go back to the driver when an allocation
-// fails; streams likewise up to kPoolStreams.  Every function may be called
-// from any thread.
+// kPoolBytes in all per device (the oldest ones go first), and go back to the
+// driver when an allocation fails; streams likewise up to kPoolStreams.  Every
+// function may be called from any thread.
+//
+// A new block is as large as what was asked for: rounded up to a power of two, a
+// 33 MB buffer needed 64 MB of free memory.  A kept block serves requests up to
+// an eighth or kPoolSlack smaller.
 constexpr size_t kPoolBlock = size_t(64) << 20;
 constexpr size_t kPoolBytes = size_t(256) << 20;
+constexpr size_t kPoolSlack = size_t(64) << 10;
 constexpr size_t kPoolStreams = 16;
-cudaError_t pool_alloc(void **ptr, size_t bytes);
+cudaError_t pool_alloc(void **ptr, size_t bytes, size_t *size);  // size: of the block
 // Inside an IdleScope whose work is done the block is kept; otherwise it is
 // freed, which waits for the device.
-void pool_free(void *ptr, size_t bytes, int device);
+void pool_free(void *ptr, size_t size, int device);
 cudaError_t pool_stream(cudaStream_t *stream);
 void pool_stream_free(cudaStream_t stream, int device);  // with no work in flight
 
