@@ -182,11 +182,13 @@ void pack_adjacency(const b200sa_problem &p, PackedAdjacency &out) {
     // 250 degree 6 4.15 -> 4.86 (not taken); random order n = 60 4.73 -> 2.00,
     // n = 120 8.16 -> 4.10, n = 250 14.6 -> 8.6.  Above 64 variables a sparse
     // problem's matrix is many times its lists, so it is made only for runs long
-    // beside its upload (2^22 attempts, about 0.1 ms).
+    // beside its upload (2^22 attempts, about 0.1 ms).  The other samplers pack
+    // a problem without a schedule and read no matrix.
     const double attempts = (double)n * p.num_reads * p.sweeps_per_beta * p.num_betas;
     const bool full = 16 * (size_t)m >= (size_t)n * (size_t)n;
     const int limit = full || p.varorder == B200SA_RANDOM ? kDenseMaxN : 128;
-    out.dense = !any_dup && n > 0 && n <= limit && (n <= 64 || full || attempts >= 4194304.0);
+    out.dense = !any_dup && attempts > 0.0 && n <= limit &&
+                (n <= 64 || full || attempts >= 4194304.0);
     out.dense_w.clear();
     if (out.dense) {
         const size_t ld = (size_t)dense_ld(n);
