@@ -40,6 +40,7 @@ EXPORTS = (
     "b200sa_plan_destroy",
     "b200sa_version",
     "b200sa_check_acceptance",
+    "b200sa_check_bounds",
     "b200sa_sample_noalloc",
     "b200sa_edge_moments",
     "b200sa_random_states",
@@ -180,9 +181,9 @@ def load() -> ctypes.CDLL:
         c.c_void_p, c.c_int32, c.POINTER(Stats), c.c_char_p, c.c_size_t]
     L.b200sa_plan_destroy.restype = c.c_int
     L.b200sa_plan_destroy.argtypes = [c.c_void_p]
-    L.b200sa_check_acceptance.restype = c.c_int
-    L.b200sa_check_acceptance.argtypes = [c.c_int64, c.c_uint64, c.c_int32, c.c_void_p,
-                                          c.c_char_p, c.c_size_t]
+    for f in (L.b200sa_check_acceptance, L.b200sa_check_bounds):
+        f.restype = c.c_int
+        f.argtypes = [c.c_int64, c.c_uint64, c.c_int32, c.c_void_p, c.c_char_p, c.c_size_t]
     L.b200sa_sample_noalloc.restype = c.c_int
     L.b200sa_sample_noalloc.argtypes = [
         c.c_int32, c.c_void_p, c.c_int64, c.c_void_p, c.c_void_p, c.c_void_p, c.c_int32,

@@ -666,8 +666,8 @@ __device__ __forceinline__ double pimc_warp_add_j4(double eff, bool first, int l
 // (errors below 2^-14 for |x| < 12, where both sides are below 35); tanh and
 // the draw then differ by more than 5e-14, far above tanh's error and the tie
 // band.  From |x| = 12 on tanh is within 1e-10 of +-1.  Inside the band the
-// exact comparison decides.  Returns the new spin, near ties in `near`.
-__device__ __forceinline__ int pimc_gibbs_draw(double x, double c, unsigned &near) {
+// exact comparison decides.  The new spin, or 0 inside the band.
+__device__ __forceinline__ int pimc_gibbs_fast(double x, double c) {
     if (fabs(x) < 12.0) {
         const float l = __fmul_rn(2.0f * kLog2e, (float)x);
         const float y = lg2_approx((float)c) - lg2_approx((float)(1.0 - c));
@@ -676,6 +676,13 @@ __device__ __forceinline__ int pimc_gibbs_draw(double x, double c, unsigned &nea
     } else if (c > 1e-9 && c < 1.0 - 1e-9 && fabs(x) < 1e300) {
         return x > 0.0 ? -1 : 1;
     }
+    return 0;
+}
+
+// The new spin, near ties in `near`.
+__device__ __forceinline__ int pimc_gibbs_draw(double x, double c, unsigned &near) {
+    const int fast = pimc_gibbs_fast(x, c);
+    if (fast) return fast;
     const double thr = __dadd_rn(__dmul_rn(c, 2.0), -1.0);  // uniform(-1, 1)
     const double t = tanh(x);
     near += fabs(t - thr) <= fabs(t) * kTieRel;

@@ -475,21 +475,32 @@ extern "C" {
 
 const char *b200sa_version(void) { return "b200sa 0.6.0 (sm_100a)"; }
 
-int b200sa_check_acceptance(int64_t samples, uint64_t seed, int32_t device,
-                            int64_t counts[6], char *err, size_t errlen) {
+static int run_check(cudaError_t (*check)(int64_t, uint64_t, unsigned long long *), int64_t samples,
+                     uint64_t seed, int32_t device, int64_t *counts, size_t size, char *err,
+                     size_t errlen) {
     if (!counts || samples < 0) return set_err(err, errlen, B200SA_EINVAL, "bad arguments");
     DeviceGuard guard;
     cudaDeviceProp prop;
     int rc = select_device(device, prop, err, errlen);
     if (rc) return rc;
     DevArray<unsigned long long> d;
-    B200SA_CUDA(d.alloc(6));
-    B200SA_CUDA(cudaMemset(d.ptr, 0, 6 * sizeof(unsigned long long)));
-    B200SA_CUDA(acceptance_check(samples, seed, d.ptr));
-    unsigned long long h[6];
-    B200SA_CUDA(cudaMemcpy(h, d.ptr, sizeof(h), cudaMemcpyDeviceToHost));
-    for (int i = 0; i < 6; ++i) counts[i] = (int64_t)h[i];
+    B200SA_CUDA(d.alloc(size));
+    B200SA_CUDA(cudaMemset(d.ptr, 0, size * sizeof(unsigned long long)));
+    B200SA_CUDA(check(samples, seed, d.ptr));
+    std::vector<unsigned long long> h(size);
+    B200SA_CUDA(cudaMemcpy(h.data(), d.ptr, size * sizeof(h[0]), cudaMemcpyDeviceToHost));
+    for (size_t i = 0; i < size; ++i) counts[i] = (int64_t)h[i];
     return B200SA_OK;
+}
+
+int b200sa_check_acceptance(int64_t samples, uint64_t seed, int32_t device,
+                            int64_t counts[6], char *err, size_t errlen) {
+    return run_check(acceptance_check, samples, seed, device, counts, 6, err, errlen);
+}
+
+int b200sa_check_bounds(int64_t samples, uint64_t seed, int32_t device, int64_t counts[9],
+                        char *err, size_t errlen) {
+    return run_check(bounds_check, samples, seed, device, counts, 9, err, errlen);
 }
 
 int b200sa_plan_create(const b200sa_problem *problems, int32_t num_problems,

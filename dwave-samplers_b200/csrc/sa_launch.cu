@@ -245,6 +245,87 @@ cudaError_t acceptance_check(int64_t samples, uint64_t seed, unsigned long long 
     return cudaGetLastError();
 }
 
+// The encoded bounds of the sweeps (Choice and draw_log2) on one decision: 1
+// flips, 0 does not, -1 left to the exact test.
+template <bool GIBBS>
+__device__ __forceinline__ int choice_fast(double d, double beta, double thr, uint64_t r) {
+    Choice<GIBBS> ch;
+    ch.look(d, Choice<GIBBS>::scale(beta), thr, true);
+    const float gap = ch.t - draw_log2(r);
+    return gap > kBand ? 1 : gap < -kBand ? 0 : -1;
+}
+
+// The same for the encoded bounds and for the path-integral Gibbs draw.  counts
+// [3 k .. 3 k + 2]: samples, decided by the bounds, decisions that differ from
+// the exact test's; k = 0 Metropolis, 1 Gibbs, 2 path integral.  Every second
+// sample lies within 2^-8 (relative) of the boundary, and there the draw is one
+// that the bounds handle (2^52 and more); three in 32 have a beta, a delta
+// energy or a draw at the ends of what they handle.
+__global__ void bounds_check_kernel(int64_t samples, uint64_t seed, unsigned long long *counts) {
+    const double betas[] = {0.0,  1e-300, 9.9e-31, 1.01e-30, 9.9e29, 1.01e30, 1e300,
+                            -1.0, 5e-324, __longlong_as_double(0x7ff0000000000000ll)};
+    const double deltas[] = {0.0, -0.0, 5e-324, -5e-324, 1e-45, 3.5e38, -3.5e38, 1e300, -1e300,
+                             __longlong_as_double(0x7ff0000000000000ll),
+                             __longlong_as_double(0xfff0000000000000ll),
+                             __longlong_as_double(0x7ff8000000000000ll)};
+    uint64_t s0 = seed ^ (0x9e3779b97f4a7c15ull * (blockIdx.x * blockDim.x + threadIdx.x + 1));
+    uint64_t s1 = 0x2545f4914f6cdd1dull;
+    for (int i = 0; i < 20; ++i) xs_next(s0, s1);
+    unsigned long long sum[9] = {};
+    auto count = [&](int k, int fast, bool exact) {
+        ++sum[3 * k];
+        if (fast < 0) return;
+        ++sum[3 * k + 1];
+        if ((fast != 0) != exact) ++sum[3 * k + 2];
+    };
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < samples;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        const uint64_t a = xs_next(s0, s1), b = xs_next(s0, s1), c = xs_next(s0, s1);
+        const uint64_t e = xs_next(s0, s1);
+        const double u = (double)(a >> 11) * 0x1p-53;  // [0, 1)
+        const double eps = ((double)(c >> 11) * 0x1p-53 - 0.5) * 0x1p-7;
+        const int odd = (int)(e & 31u);
+        const double beta = odd == 0 ? betas[(e >> 5) % 10u]
+                                     : exp(-14.0 + 28.0 * ((double)(e >> 11) * 0x1p-53));
+        const double thr = __ddiv_rn(44.36142, beta);
+        const bool at = (b & 1u) != 0;  // at the boundary
+        auto draw = [&](double t) {
+            if (odd == 2) return (uint64_t(1) << 52) + (b >> 44) - (uint64_t(1) << 19);
+            if (!at) return b;
+            t *= 1.0 + eps;
+            return t >= kTwo64 ? ~uint64_t(0) : (uint64_t)t;
+        };
+        {  // Metropolis: up to the threshold and a little beyond, and some downhill
+            const double x = (odd & 7) == 3 ? -44.35 - 0.02 * u : 0.1 - (at ? 8.5 : 44.5) * u;
+            const double d = odd == 1 ? deltas[(e >> 5) % 12u] : __ddiv_rn(-x, beta);
+            const uint64_t r = draw(exp(x) * kTwo64);
+            const bool exact = !(d >= thr) && (d <= 0.0 || (metropolis_exact(d, beta, r) & 1));
+            count(0, choice_fast<false>(d, beta, thr, r), exact);
+        }
+        {  // Gibbs
+            const double z = (odd & 7) == 3 ? 44.35 + 0.02 * u : at ? -8.0 + 16.4 * u : -30.0 + 74.4 * u;
+            const double d = odd == 1 ? deltas[(e >> 5) % 12u] : __ddiv_rn(z, beta);
+            const uint64_t r = draw(kTwo64 / (1.0 + exp(z)));
+            const bool exact = !(d >= thr) && (gibbs_exact(d, beta, r) & 1);
+            count(1, choice_fast<true>(d, beta, thr, r), exact);
+        }
+        {  // path integral: tanh(x) > 2 q - 1
+            const double x = odd == 1 ? deltas[(e >> 5) % 12u] : -12.5 + 25.0 * u;
+            double q = (double)(b >> 11) * 0x1p-53;
+            if (at) q = fmin(1.0 / (1.0 + exp(-2.0 * x) * (1.0 + eps)), 1.0 - 0x1p-53);
+            const int s = pimc_gibbs_fast(x, q);
+            const bool exact = tanh(x) > __dadd_rn(__dmul_rn(q, 2.0), -1.0);
+            count(2, s == 0 ? -1 : s < 0, exact);
+        }
+    }
+    for (int k = 0; k < 9; ++k) atomicAdd(&counts[k], sum[k]);
+}
+
+cudaError_t bounds_check(int64_t samples, uint64_t seed, unsigned long long *d_counts) {
+    bounds_check_kernel<<<148 * 4, 256>>>(samples, seed, d_counts);
+    return cudaGetLastError();
+}
+
 // arena[dst[i]] = (i < num_j ? J[src[i]] : h[src[i]]): the coupler weights
 // (adjacency entries, COO copy, back-neighbour copies) and the fields of
 // every problem of a plan, from the concatenated inputs.

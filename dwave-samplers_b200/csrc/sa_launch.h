@@ -80,5 +80,6 @@ cudaError_t launch_pimc(bool chain_update, const PimcArgs &args, int grid, int b
 cudaError_t launch_pimc_warp(const PimcArgs &args, int grid, int warps_per_cta, int warp_bytes,
                              cudaStream_t stream);
 cudaError_t acceptance_check(int64_t samples, uint64_t seed, unsigned long long *d_counts);
+cudaError_t bounds_check(int64_t samples, uint64_t seed, unsigned long long *d_counts);
 
 }  // namespace b200sa

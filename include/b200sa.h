@@ -415,9 +415,15 @@ B200SA_API int b200sa_sample_noalloc(
  * single-precision acceptance bounds used before the exact double-precision
  * test never disagree with it.  counts[6] = Metropolis {samples, decided by
  * the bounds, disagreements}, Gibbs {samples, decided by the bounds,
- * disagreements}; both disagreement counts must be 0. */
+ * disagreements}; both disagreement counts must be 0.  These are the bounds of
+ * random order outside registers and of rotor annealing. */
 B200SA_API int b200sa_check_acceptance(int64_t samples, uint64_t seed, int32_t device,
                                        int64_t counts[6], char *err, size_t errlen);
+
+/* The same for the bounds of sequential sweeps and of states in registers
+ * (Metropolis, then Gibbs) and of path-integral annealing: three counts each. */
+B200SA_API int b200sa_check_bounds(int64_t samples, uint64_t seed, int32_t device,
+                                   int64_t counts[9], char *err, size_t errlen);
 
 /* Version string of this library. */
 B200SA_API const char *b200sa_version(void);
