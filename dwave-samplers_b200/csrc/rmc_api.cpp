@@ -164,14 +164,13 @@ extern "C" int b200sa_rotor_anneal(int32_t num_vars, const double *h, int64_t nu
     a.cos_table = dtab.ptr;
     a.sin_table = dtab.ptr + 256;
     a.near = dnear.ptr;
-    // One warp per sample, or one thread with very many samples of the
-    // proposals that keep no delta energies (see rmc_kernel.cuh).  A warp's
-    // state is on chip while that keeps 12 warps per SM, or a warp for every
-    // sample; otherwise delta energies, and last the angles, go to per-warp
-    // global slots.  At equal residency the widest CTA is taken, narrower ones
-    // only to spread few samples over every SM.
+    // One warp per sample, or one thread (rmc_thread_samples).  A warp's state
+    // is on chip while that keeps 12 warps per SM, or a warp for every sample;
+    // otherwise delta energies, and last the angles, go to per-warp global
+    // slots.  At equal residency the widest CTA is taken, narrower ones only to
+    // spread few samples over every SM.
     const bool random = randomize_order != 0;
-    const bool threads = proposal >= 2 && !shared && (int64_t)R > kRmcThreadSamples;
+    const bool threads = !shared && (int64_t)R > rmc_thread_samples(proposal, random, num_vars);
     const int sms = prop.multiProcessorCount;
     const int64_t chains = shared ? 1 : (int64_t)R;
     // (A bitmap of more than 256 Ki variables stays in global memory.)
@@ -179,7 +178,9 @@ extern "C" int b200sa_rotor_anneal(int32_t num_vars, const double *h, int64_t nu
     const int touch_region = a.touch_bytes <= 32 * 1024 ? a.touch_bytes : 0;
     if (threads) {
         B200SA_CUDA(dst.alloc(n * R));
+        if (proposal <= 1) B200SA_CUDA(dde.alloc(n * R));
         a.states = dst.ptr;
+        a.de = dde.ptr;
         B200SA_CUDA(launch_rmc_thread(random, proposal, a, nullptr));
     } else {
         int stage = kStageGlobal, width = 1, ctas = 1;

@@ -20,15 +20,14 @@
 //   order each lane takes one stream position as the start of a possible
 //   attempt, as in sweep_random.
 //
-// With one thread per sample an attempt of a chain takes 2 to 3 microseconds
-// whatever the number of samples, up to about 20,000 of them.  Measured, n =
-// 512 6-regular, 64 sweeps: 4096 samples of reflections 67.5 ms with one
-// thread per sample, 5.3 ms with a warp; 32768 samples (32 sweeps) 55.8 against
-// 20.4 ms; 1000 samples of transverse-field proposals 44.8 against 5.8 ms.
-// The angle proposals spend about 30 lanes on 7 attempts, so above
-// kRmcThreadSamples samples they run one thread per sample
-// (rmc_thread_kernel): 16 sweeps of 32768 samples 12.1 ms against 19.9 with a
-// warp, of 8192 samples 11.9 against 5.5.
+// With one thread per sample (rmc_thread_kernel) an attempt of a chain takes 0.5
+// to 3 microseconds, by where its state lies, whatever the number of samples up
+// to about 20,000 of them.  Measured, n = 512 6-regular, 64 sweeps: 4096 samples
+// of reflections 67.5 ms with one thread per sample, 5.3 ms with a warp; 32768
+// samples (32 sweeps) 55.8 against 20.4 ms; 1000 samples of transverse-field
+// proposals 44.8 against 5.8 ms.  With few variables or very many samples the
+// thread is the faster one (n = 9, 262144 samples, 111 sweeps of reflections:
+// 4.2 ms against 38.7, random order 6.2 against 109): rmc_thread_samples.
 //
 // Arithmetic follows cpu_rotormc.cpp operation for operation:
 //   local field (:46-60)       h + cos(theta_nb) * J, adjacency order
@@ -532,10 +531,9 @@ __launch_bounds__(32 * kRmcMaxWarps, (kRmcCtas<RANDOM_ORDER, PROPOSAL, STAGE>))
     if (W.near && lane == 0) atomicAdd(A.near, (unsigned long long)W.near);
 }
 
-// One thread per sample, for the uniform (2) and transverse-field (3)
-// proposals with very many samples.  Angles are interleaved across samples
-// (element (v, r) at v * num_samples + r), so in sequential order a warp's 32
-// samples touch one variable in one transaction.
+// One thread per sample (see above).  Angles and delta energies are interleaved
+// across samples (element (v, r) at v * num_samples + r), so in sequential order
+// a warp's 32 samples touch one variable in one transaction.
 template <bool RANDOM_ORDER, int PROPOSAL>
 __global__ void __launch_bounds__(64) rmc_thread_kernel(RmcArgs A) {
     __shared__ double cs[256], sn[256];
@@ -553,33 +551,63 @@ __global__ void __launch_bounds__(64) rmc_thread_kernel(RmcArgs A) {
     unsigned near = 0;
     uint64_t s0 = A.seeds[r] ? A.seeds[r] : ~0ull, s1 = 0;  // cpu_rotormc.cpp:389-390
     uint8_t *st = A.states + r;  // element v at st[v * R]
+    double *de = PROPOSAL <= 1 ? A.de + r : nullptr;
     uint8_t *row = A.rows + r * n;
     for (int v = 0; v < n; ++v) st[v * R] = row[v];
+    auto field = [&](int var) {
+        const uint2 vi = __ldg(&A.vinfo[var]);
+        double e = __ldg(&A.h[var]);
+        for (unsigned k = vi.x; k < vi.x + vi.y; ++k)
+            e = __dadd_rn(e, __dmul_rn(cs[st[(int64_t)__ldg(&A.col[k]) * R]], __ldg(&A.w[k])));
+        return e;
+    };
+    if constexpr (PROPOSAL <= 1) {
+        for (int v = 0; v < n; ++v)
+            de[v * R] = __dmul_rn(field(v), __dmul_rn(-2.0, cs[st[v * R]]));
+    }
     for (int i = 0; i < 32; ++i) xs_advance(s0, s1);  // burn-in
     uint8_t *stats = A.stats ? A.stats + r * points * n : nullptr;
     for (int b = 0; b < A.num_betas; ++b) {
-        const RmcProposal q = rmc_proposal<PROPOSAL>(__ldg(&A.hp[b]), __ldg(&A.hd[b]));
+        const double beta = __ldg(&A.hp[b]);
+        [[maybe_unused]] RmcProposal q;
+        if constexpr (PROPOSAL >= 2) q = rmc_proposal<PROPOSAL>(beta, __ldg(&A.hd[b]));
         for (int sw = 0; sw < A.sweeps_per_beta; ++sw) {
             for (int i = 0; i < n; ++i) {
                 const int var = RANDOM_ORDER ? mod_n(xs_next(s0, s1), (uint32_t)n, magic) : i;
                 const uint8_t cur = st[var * R];
-                const uint64_t r1 = xs_next(s0, s1);
-                const uint64_t r2 = q.tf ? xs_next(s0, s1) : 0;
-                const uint8_t prop = rmc_angle(q, cur, r1, r2);
-                const uint2 vi = __ldg(&A.vinfo[var]);
-                double e = __ldg(&A.h[var]);
-                for (unsigned k = vi.x; k < vi.x + vi.y; ++k)
-                    e = __dadd_rn(e, __dmul_rn(cs[st[(int64_t)__ldg(&A.col[k]) * R]],
-                                               __ldg(&A.w[k])));
-                const double dlm = rmc_log_ratio(q, e, __ldg(&A.tf[var]), cs[prop], cs[cur],
-                                                 sn[prop], sn[cur]);
-                bool flip = dlm >= 0.0;
-                if (!flip) {
-                    const int x = rmc_metropolis(dlm, xs_next(s0, s1));
-                    flip = (x & 1) != 0;
+                if constexpr (PROPOSAL <= 1) {  // :167-196
+                    const double d = de[var * R];
+                    int x = 1;
+                    if (PROPOSAL == 0)
+                        x = rmc_gibbs(__dmul_rn(d, beta), xs_next(s0, s1));
+                    else if (!(d <= 0.0))
+                        x = rmc_metropolis(__dmul_rn(-d, beta), xs_next(s0, s1));
                     near += (unsigned)x >> 1;
+                    if (!(x & 1)) continue;
+                    const uint8_t prop = (uint8_t)(128 + cur);  // :270-283
+                    const double mult = __dmul_rn(2.0, __dsub_rn(cs[cur], cs[prop]));
+                    const uint2 vi = __ldg(&A.vinfo[var]);
+                    for (unsigned k = vi.x; k < vi.x + vi.y; ++k) {
+                        const int64_t nb = (int64_t)__ldg(&A.col[k]) * R;
+                        de[nb] = __dadd_rn(
+                            de[nb], __dmul_rn(__dmul_rn(mult, __ldg(&A.w[k])), cs[st[nb]]));
+                    }
+                    st[var * R] = prop;
+                    de[var * R] = -d;
+                } else {
+                    const uint64_t r1 = xs_next(s0, s1);
+                    const uint64_t r2 = q.tf ? xs_next(s0, s1) : 0;
+                    const uint8_t prop = rmc_angle(q, cur, r1, r2);
+                    const double dlm = rmc_log_ratio(q, field(var), __ldg(&A.tf[var]), cs[prop],
+                                                     cs[cur], sn[prop], sn[cur]);
+                    bool flip = dlm >= 0.0;
+                    if (!flip) {
+                        const int x = rmc_metropolis(dlm, xs_next(s0, s1));
+                        flip = (x & 1) != 0;
+                        near += (unsigned)x >> 1;
+                    }
+                    if (flip) st[var * R] = prop;
                 }
-                if (flip) st[var * R] = prop;
             }
         }
         if (stats && b % A.interval == 0) {

@@ -460,11 +460,13 @@ cudaError_t launch_rmc(bool random_order, int proposal, int stage, const RmcArgs
 
 cudaError_t launch_rmc_thread(bool random_order, int proposal, const RmcArgs &args,
                               cudaStream_t stream) {
-    static const RmcKernel table[2][2] = {{rmc_thread_kernel<false, 2>, rmc_thread_kernel<false, 3>},
-                                          {rmc_thread_kernel<true, 2>, rmc_thread_kernel<true, 3>}};
-    if (proposal != 2 && proposal != 3) return cudaErrorInvalidValue;
+    static const RmcKernel table[2][4] = {{rmc_thread_kernel<false, 0>, rmc_thread_kernel<false, 1>,
+                                           rmc_thread_kernel<false, 2>, rmc_thread_kernel<false, 3>},
+                                          {rmc_thread_kernel<true, 0>, rmc_thread_kernel<true, 1>,
+                                           rmc_thread_kernel<true, 2>, rmc_thread_kernel<true, 3>}};
+    if (proposal < 0 || proposal > 3) return cudaErrorInvalidValue;
     const int64_t grid = ((int64_t)args.num_samples + 63) / 64;
-    table[random_order ? 1 : 0][proposal - 2]<<<(unsigned)grid, 64, 0, stream>>>(args);
+    table[random_order ? 1 : 0][proposal]<<<(unsigned)grid, 64, 0, stream>>>(args);
     return cudaGetLastError();
 }
 

@@ -205,9 +205,32 @@ struct RmcArgs {
 // energies (proposals that keep them) and angles.
 constexpr int kRmcTableBytes = 2 * 256 * 8;
 constexpr int kRmcMaxWarps = 8;  // warps per CTA
-// Above this many samples the uniform and transverse-field proposals run one
-// thread per sample (both sides measured, see rmc_kernel.cuh).
-constexpr int64_t kRmcThreadSamples = 16384;
+// Above this many samples rotor annealing runs one thread per sample (all
+// proposals; per-sample streams).  A thread's time per attempt hardly grows until
+// the samples fill the chip, a warp's grows with the samples from about 12 warps
+// per SM on, and a warp's windows are mostly empty when there are few variables.
+// Both sides measured as whole calls, 1000 attempts a sample, degree 4 (ms, warp
+// against thread), n from 5 to 1024 and 1024 to 262144 samples, and degrees 3, 8
+// and 20; the line lies where they meet or a little to the warp's side:
+//   reflections, sequential  n = 16: 4096 samples 0.88, 0.82; n = 32: 8192 1.07,
+//     0.90; n = 128: 16384 1.49, 1.60, 65536 4.9, 3.3; n = 256: 65536 6.4, 6.4
+//   reflections, random      n = 32: 2048 1.20, 1.32, 4096 2.1, 1.35; n = 64: 4096
+//     1.54, 1.37; n = 128: 16384 3.0, 3.8, 65536 10.0, 6.4; n = 256: 65536 10.4, 11.9
+//   angles, sequential       n = 32: 4096 1.06, 1.08; n = 256: 8192 1.60, 1.62; n =
+//     1024: 16384 8.4, 8.1
+//   angles, random           n = 32: 2048 1.45, 1.53; n = 64: 4096 1.88, 1.56; n =
+//     256: 8192 2.26, 2.05; n = 512: 16384 6.7, 9.3, 32768 12.2, 11.1
+// Beyond 128 variables a thread's delta energies leave the caches.
+inline int64_t rmc_thread_samples(int proposal, bool random_order, int n) {
+    const int64_t never = INT32_MAX;
+    if (proposal <= 1) {
+        if (n > 128) return never;
+        if (!random_order) return n <= 16 ? 4096 : 256 * (int64_t)n;
+        return n <= 32 ? 2560 : n <= 64 ? 80 * (int64_t)n : 32768;
+    }
+    if (!random_order) return 4096 + 16 * (int64_t)n;
+    return n <= 53 ? 2560 : n <= 256 ? 48 * (int64_t)n : 64 * (int64_t)n;
+}
 
 // Arguments of the path-integral Monte Carlo kernel (pimc_kernel.cuh).  One
 // thread per sample (a "slot"); every slot owns an mt19937 state and a
