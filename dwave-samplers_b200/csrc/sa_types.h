@@ -141,12 +141,12 @@ struct SdArgs {
     double *energies;
     uint32_t *steps;
     uint32_t max_steps;
-    int32_t smem_cap_n;          // state in shared memory when > 0
-    double *scratch_fe;          // else per-warp global slots
+    double *scratch_fe;          // per-warp global slots, or null: state in shared memory
     int8_t *scratch_s;
     int64_t scratch_stride;
     int32_t table_bytes;         // list starts at the head of a CTA's shared memory
     int32_t any_dup;             // some list names a target twice
+    int32_t flat;                // no group minima: every step looks at all variables
     unsigned long long *scratch_key;  // group minima (sd_kernel.cuh)
     uint8_t *scratch_at;
     int64_t group_stride;
@@ -164,6 +164,15 @@ inline int64_t sd_region_bytes(int64_t cap_n) {
     const int64_t groups = (cap_n + 31) / 32;
     return (kSdScratchBytes + 8 * (cap_n + groups) + cap_n + groups + 15) & ~int64_t(15);
 }
+
+// Whether a step looks at every variable instead of the group minima: with few
+// groups, and where a flip's list is long enough to change most of them (mean
+// degree n / 12 and more).  Group minima against all variables, whole calls of
+// 8192 samples (ms): n = 128 degree 6 0.93, 0.91; n = 300 degree 3 1.30, 1.32,
+// degree 50 2.64, 2.45, complete 12.0, 11.0; n = 500 degree 25 2.69, 2.78, degree
+// 50 4.08, 3.86; n = 1000 degree 50 7.98, 8.42, degree 100 14.1, 13.5; n = 2048
+// degree 6 7.7, 13.0, degree 100 33.3, 33.2, degree 200 62.3, 56.4.
+inline bool sd_flat(int64_t n, int64_t m) { return n <= 256 || 24 * m >= n * n; }
 
 // Arguments of the rotor-model annealing kernel (rmc_kernel.cuh).
 struct RmcArgs {

@@ -86,7 +86,6 @@ extern "C" int b200sa_steepest_descent(int32_t num_vars, const double *h, int64_
             break;
         onchip = false;
     }
-    const int cap = onchip ? num_vars : 0;
     if (best == 0) return set_err(err, errlen, B200SA_ECUDA, "descent kernel does not fit");
     const int w = (int)std::min<int64_t>(best_w, std::max<int64_t>(1, (num_samples + sms - 1) / sms));
     int ctas = 0;
@@ -127,12 +126,12 @@ extern "C" int b200sa_steepest_descent(int32_t num_vars, const double *h, int64_
     a.energies = den.ptr;
     a.steps = dsteps.ptr;
     a.max_steps = max_steps;
-    a.smem_cap_n = cap;
     a.scratch_fe = sfe.ptr;
     a.scratch_s = ss.ptr;
     a.scratch_stride = stride;
     a.table_bytes = table;
     a.any_dup = plan->any_dup ? 1 : 0;
+    a.flat = sd_flat(num_vars, num_couplers) ? 1 : 0;
     a.scratch_key = gkey.ptr;
     a.scratch_at = gat.ptr;
     a.group_stride = groups;

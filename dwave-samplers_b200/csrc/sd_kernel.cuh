@@ -33,7 +33,9 @@ namespace b200sa {
 // = 2048, 6-regular; this takes 3.9 ms.  What is left is the latency of a step,
 // about 1700 cycles: the list from L2, three reductions each for the least
 // group and for the flipped group.  Fetching the list of the next group minimum
-// ahead gained nothing: its reductions cost what it saved.)
+// ahead gained nothing: its reductions cost what it saved.)  With few groups, or
+// lists so long that a flip leaves few groups as they were, a step looks at all
+// variables instead (SdArgs::flat, sd_flat).
 //
 // A key orders negative energies (more negative is smaller); every other value,
 // NaN included, is kSdNone, never chosen.
@@ -118,7 +120,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1)
         const int r = (int)(A.items[it] & 0xffffffffll);
         const int64_t so = PD->state_offset + (int64_t)r * n;
         load_state(PD, A.states_in + so, fe, sp, lane);  // descent.cpp:41-60, 128-133
-        for (int g = 0; g < groups; ++g) G.scan(fe, g, n, lane);
+        for (int g = 0; g < groups && !A.flat; ++g) G.scan(fe, g, n, lane);
         __syncwarp();
         uint32_t steps = 0;
         bool capped = false;
@@ -127,11 +129,22 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1)
             // ties to the lowest index.
             unsigned long long bk = kSdNone;
             unsigned best = ~0u;
-            for (int g = (int)lane; g < groups; g += 32) {
-                const unsigned long long k = G.key[g];
-                if (k < bk) {
-                    bk = k;
-                    best = 32u * (unsigned)g + G.at[g];
+            if (A.flat) {
+#pragma unroll 4
+                for (int v = (int)lane; v < n; v += 32) {
+                    const unsigned long long k = sd_key(fe[v]);
+                    if (k < bk) {
+                        bk = k;
+                        best = (unsigned)v;
+                    }
+                }
+            } else {
+                for (int g = (int)lane; g < groups; g += 32) {
+                    const unsigned long long k = G.key[g];
+                    if (k < bk) {
+                        bk = k;
+                        best = 32u * (unsigned)g + G.at[g];
+                    }
                 }
             }
             warp_least(bk, best);
@@ -196,6 +209,8 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1)
                 fe[bv] = __dmul_rn(be, -1.0);
             }
             __syncwarp();
+            ++steps;
+            if (A.flat) continue;
             // Groups whose minimum may have changed: the flipped variable's,
             // and those where a neighbour was it or falls below it.
             G.scan(fe, bv >> 5, n, lane);
@@ -219,7 +234,6 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1)
                 }
                 __syncwarp();
             }
-            ++steps;
         }
         __syncwarp();
         const double e = state_energy(PD, sp, scratch, lane);  // descent.cpp:75-93
