@@ -400,14 +400,18 @@ cudaError_t kernel_occupancy(int variant, int warps_per_cta, int region_bytes, i
 
 using SdKernel = void (*)(SdArgs, int, int);
 
-static SdKernel sd_kernel_for(bool sparse, bool smem) {
-    if (sparse) return smem ? sd_warp_kernel<true, true> : sd_warp_kernel<true, false>;
-    return smem ? sd_warp_kernel<false, true> : sd_warp_kernel<false, false>;
+static SdKernel sd_kernel_for(bool sparse, bool smem, bool flat) {
+    static const SdKernel table[2][2][2] = {
+        {{sd_warp_kernel<false, false, false>, sd_warp_kernel<false, false, true>},
+         {sd_warp_kernel<false, true, false>, sd_warp_kernel<false, true, true>}},
+        {{sd_warp_kernel<true, false, false>, sd_warp_kernel<true, false, true>},
+         {sd_warp_kernel<true, true, false>, sd_warp_kernel<true, true, true>}}};
+    return table[sparse][smem][flat];
 }
 
-cudaError_t launch_sd(bool sparse, bool smem, const SdArgs &args, int grid, int warps_per_cta,
-                      int region_bytes, cudaStream_t stream) {
-    const SdKernel k = sd_kernel_for(sparse, smem);
+cudaError_t launch_sd(bool sparse, bool smem, bool flat, const SdArgs &args, int grid,
+                      int warps_per_cta, int region_bytes, cudaStream_t stream) {
+    const SdKernel k = sd_kernel_for(sparse, smem, flat);
     const size_t bytes = (size_t)args.table_bytes + (size_t)warps_per_cta * (size_t)region_bytes;
     cudaError_t e = open_smem(k);
     if (e != cudaSuccess) return e;
@@ -415,9 +419,9 @@ cudaError_t launch_sd(bool sparse, bool smem, const SdArgs &args, int grid, int 
     return cudaGetLastError();
 }
 
-cudaError_t sd_occupancy(bool sparse, bool smem, int warps_per_cta, int region_bytes,
+cudaError_t sd_occupancy(bool sparse, bool smem, bool flat, int warps_per_cta, int region_bytes,
                          int table_bytes, int *ctas_per_sm) {
-    const SdKernel k = sd_kernel_for(sparse, smem);
+    const SdKernel k = sd_kernel_for(sparse, smem, flat);
     const size_t bytes = (size_t)table_bytes + (size_t)warps_per_cta * (size_t)region_bytes;
     cudaError_t e = open_smem(k);
     if (e != cudaSuccess) return e;

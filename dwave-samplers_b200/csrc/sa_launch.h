@@ -61,9 +61,9 @@ cudaError_t launch_sa(int variant, const LaunchArgs &args, int grid, int warps_p
                       int region_bytes, cudaStream_t stream);
 cudaError_t kernel_occupancy(int variant, int warps_per_cta, int region_bytes,
                              int *ctas_per_sm);
-cudaError_t launch_sd(bool sparse, bool smem, const SdArgs &args, int grid, int warps_per_cta,
-                      int region_bytes, cudaStream_t stream);
-cudaError_t sd_occupancy(bool sparse, bool smem, int warps_per_cta, int region_bytes,
+cudaError_t launch_sd(bool sparse, bool smem, bool flat, const SdArgs &args, int grid,
+                      int warps_per_cta, int region_bytes, cudaStream_t stream);
+cudaError_t sd_occupancy(bool sparse, bool smem, bool flat, int warps_per_cta, int region_bytes,
                          int table_bytes, int *ctas_per_sm);
 // Rotor kernel; `stage` is its state location (kStageShared only for the
 // proposals that keep delta energies, 0 and 1).

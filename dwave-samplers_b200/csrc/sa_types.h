@@ -146,7 +146,6 @@ struct SdArgs {
     int64_t scratch_stride;
     int32_t table_bytes;         // list starts at the head of a CTA's shared memory
     int32_t any_dup;             // some list names a target twice
-    int32_t flat;                // no group minima: every step looks at all variables
     unsigned long long *scratch_key;  // group minima (sd_kernel.cuh)
     uint8_t *scratch_at;
     int64_t group_stride;

@@ -57,7 +57,7 @@ extern "C" int b200sa_steepest_descent(int32_t num_vars, const double *h, int64_
     std::unique_ptr<b200sa_plan_s, void (*)(b200sa_plan)> hold(plan, release_plan);
     DeviceGuard guard;
     B200SA_CUDA(cudaSetDevice(plan->device));
-    const bool sparse = large_sparse_opt != 0;
+    const bool sparse = large_sparse_opt != 0, flat = sd_flat(num_vars, num_couplers);
     const int smem_blk = (int)plan->prop.sharedMemPerBlockOptin;
     const int sms = plan->prop.multiProcessorCount;
     // State in shared memory while that keeps 10 warps per SM, or two rounds of
@@ -76,7 +76,7 @@ extern "C" int b200sa_steepest_descent(int32_t num_vars, const double *h, int64_
         for (int w = 1; w <= kMaxThreadsPerCta / 32 && (int64_t)table + w * (int64_t)region <= smem_blk;
              ++w) {
             int ctas = 0;
-            B200SA_CUDA(sd_occupancy(sparse, onchip, w, region, table, &ctas));
+            B200SA_CUDA(sd_occupancy(sparse, onchip, flat, w, region, table, &ctas));
             if (ctas * w > best) {
                 best = ctas * w;
                 best_w = w;
@@ -89,7 +89,7 @@ extern "C" int b200sa_steepest_descent(int32_t num_vars, const double *h, int64_
     if (best == 0) return set_err(err, errlen, B200SA_ECUDA, "descent kernel does not fit");
     const int w = (int)std::min<int64_t>(best_w, std::max<int64_t>(1, (num_samples + sms - 1) / sms));
     int ctas = 0;
-    B200SA_CUDA(sd_occupancy(sparse, onchip, w, region, table, &ctas));
+    B200SA_CUDA(sd_occupancy(sparse, onchip, flat, w, region, table, &ctas));
     const int grid = (int)std::max<int64_t>(
         1, std::min<int64_t>((int64_t)sms * std::max(ctas, 1), (num_samples + w - 1) / w));
     const int64_t slots = (int64_t)grid * w;
@@ -131,12 +131,11 @@ extern "C" int b200sa_steepest_descent(int32_t num_vars, const double *h, int64_
     a.scratch_stride = stride;
     a.table_bytes = table;
     a.any_dup = plan->any_dup ? 1 : 0;
-    a.flat = sd_flat(num_vars, num_couplers) ? 1 : 0;
     a.scratch_key = gkey.ptr;
     a.scratch_at = gat.ptr;
     a.group_stride = groups;
     a.capped = counters.ptr + 1;
-    B200SA_CUDA(launch_sd(sparse, onchip, a, grid, w, region, st));
+    B200SA_CUDA(launch_sd(sparse, onchip, flat, a, grid, w, region, st));
     unsigned long long capped = 0;
     B200SA_CUDA(cudaMemcpyAsync(states, dstates.ptr, total, cudaMemcpyDeviceToHost, st));
     B200SA_CUDA(cudaMemcpyAsync(energies, den.ptr, sizeof(double) * (size_t)num_samples,

@@ -35,7 +35,7 @@ namespace b200sa {
 // group and for the flipped group.  Fetching the list of the next group minimum
 // ahead gained nothing: its reductions cost what it saved.)  With few groups, or
 // lists so long that a flip leaves few groups as they were, a step looks at all
-// variables instead (SdArgs::flat, sd_flat).
+// variables instead (FLAT, sd_flat).
 //
 // A key orders negative energies (more negative is smaller); every other value,
 // NaN included, is kSdNone, never chosen.
@@ -70,7 +70,7 @@ struct SdGroups {
     }
 };
 
-template <bool SPARSE, bool SMEM>
+template <bool SPARSE, bool SMEM, bool FLAT>
 __global__ void __launch_bounds__(kMaxThreadsPerCta, 1)
     sd_warp_kernel(SdArgs A, int warps_per_cta, int region_bytes) {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1)
         const int r = (int)(A.items[it] & 0xffffffffll);
         const int64_t so = PD->state_offset + (int64_t)r * n;
         load_state(PD, A.states_in + so, fe, sp, lane);  // descent.cpp:41-60, 128-133
-        for (int g = 0; g < groups && !A.flat; ++g) G.scan(fe, g, n, lane);
+        for (int g = 0; !FLAT && g < groups; ++g) G.scan(fe, g, n, lane);
         __syncwarp();
         uint32_t steps = 0;
         bool capped = false;
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1)
             // ties to the lowest index.
             unsigned long long bk = kSdNone;
             unsigned best = ~0u;
-            if (A.flat) {
+            if constexpr (FLAT) {
 #pragma unroll 4
                 for (int v = (int)lane; v < n; v += 32) {
                     const unsigned long long k = sd_key(fe[v]);
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(kMaxThreadsPerCta, 1)
             }
             __syncwarp();
             ++steps;
-            if (A.flat) continue;
+            if (FLAT) continue;
             // Groups whose minimum may have changed: the flipped variable's,
             // and those where a neighbour was it or falls below it.
             G.scan(fe, bv >> 5, n, lane);
