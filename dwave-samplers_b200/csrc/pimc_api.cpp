@@ -31,6 +31,13 @@ int auto_capacity(const double *hd, int num_betas) {
     return (int)std::min(1e6, std::ceil(cap / 4.0) * 4.0);
 }
 
+// The transverse field's mean over the schedule (for pimc_thread_samples).
+double mean_field(const double *hd, int num_betas) {
+    double sum = 0.0;
+    for (int b = 0; b < num_betas; ++b) sum += std::isfinite(hd[b]) ? std::fabs(hd[b]) : 0.0;
+    return num_betas ? sum / num_betas : 0.0;
+}
+
 }  // namespace
 
 extern "C" int b200sa_path_anneal(
@@ -107,10 +114,12 @@ extern "C" int b200sa_path_anneal(
     const int cap_breaks = std::max(cap_props, (max_in + 3) & ~3);
     // Single-qubit updates run on a warp per sample while a CTA's warps fit in
     // shared memory; chain updates, very large capacities, break lists out of
-    // order and more than kPimcThreadSamples samples on one thread per sample.
+    // order and more than pimc_thread_samples samples on one thread per sample.
     const int64_t warp_bytes = pimc_warp_bytes(cap_props, cap_breaks);
     const bool warp = !chain && ordered && warp_bytes <= 48 * 1024 &&
-                      (num_seeds == 1 || num_samples <= kPimcThreadSamples);
+                      (num_seeds == 1 ||
+                       num_samples <= pimc_thread_samples(num_vars, num_couplers,
+                                                          mean_field(hd_field, num_betas)));
     const int Q = chain ? qubits_per_chain : 1;
     const int64_t C = (int64_t)cap_props + cap_breaks;
     // props, itf [Q][C], sv [Q * C], off [Q + 1], lab [Q * C], parent [Q * C], pair [2C]

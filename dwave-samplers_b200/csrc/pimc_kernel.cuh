@@ -6,9 +6,9 @@
 // one Gibbs draw per domain) from one mt19937 stream and merges variable-length
 // break lists, so a sample is one sequential chain of updates, bound by the
 // latency of one update; many samples run side by side.  Single-qubit updates
-// run on a warp per sample (pimc_warp_kernel, below), chain updates,
-// unusual inputs and calls of very many samples on one thread per sample.  Every sample keeps its
-// world lines in global memory: the first Trotter slice (int8 spins), the
+// run on a warp per sample (pimc_warp_kernel, below), chain updates, unusual
+// inputs and calls of very many samples on one thread per sample.  Every sample
+// keeps its world lines in global memory: the first Trotter slice (int8 spins), the
 // number of breaks of each variable and their positions (cap_breaks slots per
 // variable, increasing).  Every slot (thread) keeps its mt19937 state and a
 // scratch area (proposals, interfaces, domain fields, chain labels).
@@ -440,11 +440,11 @@ __global__ void __launch_bounds__(64) pimc_kernel(PimcArgs A) {
 // and whose spin they draw.  An update takes about 900 warp instructions, which
 // is what bounds it: 6 cycles each for few samples (with one thread per sample
 // the latency of dependent loads, about 50,000 cycles an update), the issue
-// slots (70% busy) from about 4000 samples on.  Measured, n = 512 6-regular, 16
-// steps, field 5 -> 0.05: 4096 samples 209 ms with one thread per sample, 118 ms
-// with four samples to a warp (8 lanes each; the samples of a warp diverge), 40
-// ms with a warp; 1000 samples (8 steps) 107 -> 15 ms, 16384 139 -> 78 ms;
-// kPimcThreadSamples is where the thread per sample becomes the faster one.
+// slots (70% busy) from about 4000 samples on.  Measured, n = 512 6-regular, field
+// 5 -> 0.05, 16 steps: 4096 samples 209 ms with one thread per sample, 118 ms with
+// four samples to a warp (8 lanes each; the samples of a warp diverge), 40 ms with
+// a warp; 8 steps: 1000 samples 107 -> 15 ms, 16384 139 -> 78 ms.  From
+// pimc_thread_samples on the thread per sample is the faster one.
 
 // mt19937 as a ring in shared memory: slot k mod 624 is replaced in place by
 // word k + 624, 32 words at a time and only a few ahead of the draws.

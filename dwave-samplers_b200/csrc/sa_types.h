@@ -1,5 +1,6 @@
 // Types shared by the host packer, the launch code and the sm_100a kernels.
 #pragma once
+#include <cmath>
 #include <cstdint>
 
 #include <vector_types.h>
@@ -188,7 +189,7 @@ struct RmcArgs {
     int32_t num_betas;
     int32_t sweeps_per_beta;
     const uint64_t *seeds;
-    int32_t shared_stream;   // 1: one thread, samples in order, one RNG stream
+    int32_t shared_stream;   // 1: one warp, samples in order, one RNG stream
     int32_t num_samples;
     uint8_t *rows;           // [num_samples][n] initial states in, final states out
     const uint8_t *dist;     // [n] speculation distance (ProblemDev::dist)
@@ -200,7 +201,7 @@ struct RmcArgs {
     uint32_t *touch;         // the bitmaps, one per warp, or null: in the region
     double *de;              // per-warp global slots of slot_stride elements
     uint8_t *states;         // (state locations kStageSpins and kStageGlobal);
-    int64_t slot_stride;     // one thread per sample: angles, [n][num_samples]
+    int64_t slot_stride;     // one thread per sample: both [n][num_samples]
     double *energies;
     uint8_t *stats;          // [num_samples][points][n], or null
     int32_t interval;
@@ -240,9 +241,9 @@ inline int64_t rmc_thread_samples(int proposal, bool random_order, int n) {
     return n <= 53 ? 2560 : n <= 256 ? 48 * (int64_t)n : 64 * (int64_t)n;
 }
 
-// Arguments of the path-integral Monte Carlo kernel (pimc_kernel.cuh).  One
-// thread per sample (a "slot"); every slot owns an mt19937 state and a
-// scratch area in global memory.  Break lists have a fixed capacity per
+// Arguments of the path-integral Monte Carlo kernels (pimc_kernel.cuh): a warp
+// per sample, mt19937 state and scratch in shared memory, or a thread per sample
+// (a "slot"), both in global memory.  Break lists have a fixed capacity per
 // variable; proposals and domains per update have one too.
 struct PimcArgs {
     int32_t n;
@@ -260,7 +261,7 @@ struct PimcArgs {
     int32_t qpc;             // qubits per chain (chain update)
     int32_t chains;          // n / qpc
     const uint32_t *seeds;
-    int32_t shared_stream;   // 1: one thread, samples in order, one generator
+    int32_t shared_stream;   // 1: one warp or thread, samples in order, one generator
     int32_t num_samples;
     int8_t *states;          // [num_samples][n], the first Trotter slice
     int32_t *counts;         // [num_samples][n] breaks per variable
@@ -268,7 +269,7 @@ struct PimcArgs {
     int32_t cap_breaks;
     int32_t list_stride;     // cap_breaks, rounded up to 16 bytes
     int32_t cap_props;       // proposals per qubit and update
-    uint32_t *mt;            // [slots][kMtWords]
+    uint32_t *mt;            // [slots][kMtWords]; null (as the scratch) for a warp per sample
     int32_t *scratch_i;      // [slots][scratch_ints]
     double *scratch_d;       // [slots][scratch_doubles]
     int64_t scratch_ints, scratch_doubles;
@@ -283,13 +284,25 @@ constexpr int kPimcSlices = 65536;  // numTrotterSlices, localPIMC.h:88
 // Warps per CTA of the warp-per-sample kernel at most, and its shared memory
 // per sample: mt19937 state, scratch (PimcWarpScratch).
 constexpr int kPimcMaxWarps = 4;
-// Above this many samples single-qubit updates run one thread per sample: the
-// threads then fill the chip, while a warp per sample already issues at its
-// limit and its time grows with the samples.  n = 512, 16 steps, field 5 ->
-// 0.05, kernel time of a warp and of a thread per sample: 151 and 249 ms with
-// 16384 samples, 288 and 315 with 32768, 566 and 497 with 65536; lines through
-// these cross near 41000.
-constexpr int64_t kPimcThreadSamples = 40960;
+// Above this many samples single-qubit updates run one thread per sample.  A
+// warp's update costs nearly the same whatever it finds; a thread's grows with
+// the domains (the transverse field, here its mean over the schedule), with the
+// neighbours and with the distance of its lists, and hardly with the samples
+// until they fill the chip.  Where the two meet, as whole calls of a field
+// falling geometrically to 0.05 (mean 0.14, 0.32 and 1.07; samples): n = 5:
+// 9000, 12500, 22500; n = 12 degree 4 12000, 16000, 36000, degree 11 14500, 18000,
+// 41000; n = 32 degree 4 14500, 19500, 42000, degree 12 20000, 28000, 62000; n =
+// 128 degree 4 18500, 33000, beyond, degree 12 33500, 50000, beyond; n = 512
+// degree 4 22500.  The product below follows these; from n = 512 on the samples'
+// lists leave the caches and the line lies near 42000 (degree 6, field 5 ->
+// 0.05, 16 steps, kernel time of a warp and of a thread: 16384 samples 151, 249
+// ms, 32768 288, 315, 65536 566, 497), so it ends there.
+inline int64_t pimc_thread_samples(int64_t n, int64_t m, double mean_field) {
+    const double degree = 2.0 * (double)m / (double)n;
+    const double line = 4350.0 * (1.0 + 2.65 * mean_field) * (1.0 + degree / 12.0) *
+                        std::pow((double)n, 1.0 / 6.0);
+    return line < 40960.0 ? (int64_t)line : 40960;
+}
 inline int64_t pimc_warp_bytes(int64_t cap_props, int64_t cap_breaks) {
     const int64_t cap = cap_props + cap_breaks;
     return (4 * kMtWords + 32 * (8 + 4 + 4) + 8 * cap + cap + 15) & ~int64_t(15);
