@@ -31,15 +31,23 @@ std::map<int, DevicePool> &device_pools() {
     return *pools;
 }
 
+size_t pool_size(size_t bytes) {
+    if (bytes > kPoolSmall) return (bytes + 511) & ~size_t(511);
+    size_t c = 512;
+    while (c < bytes) c <<= 1;
+    return c;
+}
+
 }  // namespace
 
 cudaError_t pool_alloc(void **ptr, size_t bytes, size_t *size) {
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
-    bytes = (bytes + 511) & ~size_t(511);
+    const size_t exact = (bytes + 511) & ~size_t(511);
+    bytes = pool_size(bytes);
     if (bytes <= kPoolBlock) {
-        const size_t most = bytes + std::max(bytes / 8, kPoolSlack);
+        const size_t most = bytes + bytes / 8;
         std::lock_guard<std::mutex> lock(g_pool_mutex);
         DevicePool &pool = device_pools()[device];
         auto best = pool.blocks.end();
@@ -67,7 +75,8 @@ cudaError_t pool_alloc(void **ptr, size_t bytes, size_t *size) {
         pool.bytes = 0;
     }
     for (const Block &b : back) cudaFree(b.ptr);
-    return cudaMalloc(ptr, bytes);
+    *size = exact;
+    return cudaMalloc(ptr, exact);
 }
 
 void pool_free(void *ptr, size_t size, int device) {

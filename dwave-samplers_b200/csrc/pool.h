@@ -15,12 +15,13 @@ namespace host {
 // driver when an allocation fails; streams likewise up to kPoolStreams.  Every
 // function may be called from any thread.
 //
-// A new block is as large as what was asked for: rounded up to a power of two, a
-// 33 MB buffer needed 64 MB of free memory.  A kept block serves requests up to
-// an eighth or kPoolSlack smaller.
+// A new block above kPoolSmall is as large as what was asked for: rounded up to
+// a power of two, a 33 MB buffer needed 64 MB of free memory.  Smaller ones are
+// rounded up, so that calls of other sizes find them, but not when memory is
+// short.  A kept block serves requests up to an eighth smaller.
 constexpr size_t kPoolBlock = size_t(64) << 20;
 constexpr size_t kPoolBytes = size_t(256) << 20;
-constexpr size_t kPoolSlack = size_t(64) << 10;
+constexpr size_t kPoolSmall = size_t(16) << 20;
 constexpr size_t kPoolStreams = 16;
 cudaError_t pool_alloc(void **ptr, size_t bytes, size_t *size);  // size: of the block
 // Inside an IdleScope whose work is done the block is kept; otherwise it is
